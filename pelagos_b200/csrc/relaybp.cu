@@ -4,8 +4,7 @@
 
 #include "relaybp.h"
 #include "relaybp_host.h"
-#include "relaybp_kernel.cuh"
-#include "relaybp_slots.cuh"
+#include "relaybp_decode.cuh"
 
 #include <cuda_runtime.h>
 
@@ -37,26 +36,40 @@ std::string& err_slot() {
 }
 }  // namespace rbph
 
+namespace {
+
+// Byte offsets of a block's shared memory.
+struct Layout {
+  int off_chk_deg, off_llr, off_first, off_group0;
+  int g_msg, g_par, g_best, g_first, g_red, g_s1, group_bytes;
+  bool sums;
+};
+
+struct Launch {
+  KernelFn kernel;
+  int group_threads, groups, blocks;
+  int nshots;  // shots per group, as configured
+  int minb;    // resident blocks per SM the kernel is compiled for
+  Layout L;
+};
+
+}  // namespace
+
 struct rbp_decoder {
   const rbp_graph* g = nullptr;
   rbp_params p{};
   int rows = 0;                // check slots per row in the layout (padded, multiple of VEC)
   DevBuf<uint16_t> var_pos;    // [vslots, V] slot index of variable v's k-th edge
+  DevBuf<uint16_t> var_chk;    // [V, chk_stride] check of variable v's k-th edge
   DevBuf<float> llr;
   DevBuf<float> gamma_legs;
   DevBuf<float> alpha;
   DevBuf<int> queue;
   int n_alpha = 0;
+  bool strict = false;         // masked check rows (strict_rows)
   // launch shapes: shape[0] for launches that skip the relay legs (pre-iterations
   // only, so a shot's latency is bounded by pre_iter), shape[1] for the others
-  struct Shape {
-    KernelFn kernel = nullptr;
-    int group_threads = 0, groups = 0, blocks = 0, vpt = 0;
-    int nshots = 1;            // shots a group decodes at once
-    int slots_kernel = 0;      // 1: relaybp_slots_kernel (one group per block)
-    int minb = 1;              // resident blocks per SM the kernel is compiled for
-    int group_bytes = 0, block_bytes = 0;
-  } shape[2];
+  Launch shape[2];
   int sm_count = 0;
   size_t max_smem = 0;
 };
@@ -64,11 +77,6 @@ struct rbp_decoder {
 namespace {
 
 size_t msg_size(int t) { return t == RBP_MSG_F64 ? 8 : (t == RBP_MSG_F32 ? 4 : 2); }
-
-struct Layout {
-  int off_chk_deg, off_llr, off_first, off_group0;
-  int g_msg, g_par, g_best, g_first, g_red, g_s1, group_bytes;
-};
 
 // Rows of the check-slot layout: the slot count the kernel holds in registers
 // (8 or 16) or the exact maximum degree, rounded up to whole 16-byte chunks.
@@ -87,11 +95,11 @@ int slot_index_host(int j, int c, int C, int msg_type) {
   }
 }
 
-// Block-wide tables first, then one region per group.  first_sums: the region also holds
-// the shot's first-pass sums and the memory mixes a relay leg's first iteration keeps for its
-// deferred stores, one accumulator each per owned-variable slot (the one-shot block-per-group
-// kernel).
-Layout make_layout(int C, int V, int rows, int msg_type, int group_threads, bool first_sums = false) {
+// Block-wide tables first, then one region per group.  vpt: owned variables per thread of
+// the kernel.  sums: the region also holds the shot's first-pass sums and the memory mixes a
+// relay leg's first iteration keeps for its deferred stores, one accumulator each per
+// owned-variable slot.
+Layout make_layout(int C, int V, int rows, int msg_type, int group_threads, int vpt, bool sums) {
   Layout L{};
   int o = 0;
   L.off_chk_deg = o;
@@ -115,17 +123,18 @@ Layout make_layout(int C, int V, int rows, int msg_type, int group_threads, bool
   L.g_red = q;
   q = align16(q + 8 * (group_threads / 32 + 4));
   L.g_s1 = q;
-  if (first_sums) {
-    int vpt = 16;  // owned variables per thread (vpt_for)
-    for (int v : rbpk::kVptChoices)
-      if ((long long)v * group_threads >= V) {
-        vpt = v;
-        break;
-      }
-    q = align16(q + (msg_type == RBP_MSG_F64 ? 8 : 4) * 2 * vpt * group_threads);  // + memory mixes
-  }
-  L.group_bytes = q;
+  L.sums = sums;
+  if (sums) q = align16(q + (msg_type == RBP_MSG_F64 ? 8 : 4) * 2 * vpt * group_threads);
+  // owned-variable slots beyond V read past the prior table (values not used): inside the block's memory
+  L.group_bytes = std::max(q, align16(L.off_llr + 4 * vpt * group_threads - L.off_group0));
   return L;
+}
+
+// The layout with the sums where `groups` groups still fit, else without.
+Layout fit_layout(int C, int V, int rows, int msg_type, int group_threads, int vpt, int groups, size_t max_smem) {
+  const Layout L = make_layout(C, V, rows, msg_type, group_threads, vpt, true);
+  if ((size_t)L.off_group0 + (size_t)groups * L.group_bytes <= max_smem) return L;
+  return make_layout(C, V, rows, msg_type, group_threads, vpt, false);
 }
 
 KernelFn pick_kernel(int msg_type, int dc, int dv, int vpt) {
@@ -138,15 +147,76 @@ KernelFn pick_kernel(int msg_type, int dc, int dv, int vpt) {
   }
 }
 
-KernelFn pick_slots_kernel(int msg_type, int dc, int dv, int vpt, int ns, int minb) {
+KernelFn pick2_kernel(int msg_type, int dc, int dv, int vpt) {
   switch (msg_type) {
-    case RBP_MSG_F32: return rbpk::pick_slots_f32(dc, dv, vpt, ns, minb);
-    case RBP_MSG_F16: return rbpk::pick_slots_f16(dc, dv, vpt, ns, minb);
-    case RBP_MSG_BF16: return rbpk::pick_slots_bf16(dc, dv, vpt, ns, minb);
-    case RBP_MSG_F64: return rbpk::pick_slots_f64(dc, dv, vpt, ns, minb);
+    case RBP_MSG_F32: return rbpk::pick2_f32(dc, dv, vpt);
+    case RBP_MSG_F16: return rbpk::pick2_f16(dc, dv, vpt);
+    case RBP_MSG_BF16: return rbpk::pick2_bf16(dc, dv, vpt);
+    case RBP_MSG_F64: return rbpk::pick2_f64(dc, dv, vpt);
     default: return nullptr;
   }
 }
+
+// Largest group that may be configured with two shots per group (the limits callers know).
+int max_two_shot_threads(int vpt) { return vpt <= 4 ? 512 : (vpt == 6 ? 480 : (vpt == 8 ? 384 : (vpt == 12 ? 256 : 192))); }
+
+int max_group_threads(int vpt, int nshots, int minb) {
+  return minb == 2 ? rbpk::max_block_threads2(vpt) : (nshots == 2 ? max_two_shot_threads(vpt) : rbpk::max_block_threads(vpt));
+}
+
+// Slot of each edge within its check's row.  A check pass does not care about the order
+// of a row's slots (a minimum and a sign product), but the variable pass does: a warp's
+// 32 variables access their k-th edges together, and two messages in different words of
+// one shared-memory bank cost a second pass.  Starting from the order of the row, pairs
+// of a row's edges trade slots while that evens out the banks of the accesses they take
+// part in.  Passes over shared memory per sweep of all variables' edges (float32): the
+// 936 x 2592 phenomenological matrix 590 -> 405 (243 without any conflict), the 2000 x
+// 4000 (3,6)-regular one 1313 -> 784 (375).
+std::vector<int> conflict_free_slots(const rbp_graph& g, int msg_type) {
+  std::vector<int> slot = g.edge_slot;
+  if (g.slots > 16 || msg_type == RBP_MSG_F64) return slot;  // 8-byte accesses go by half warps: left alone
+  const int K = g.vslots, groups = (g.V + 31) / 32 * K, words = (int)msg_size(msg_type);
+  std::vector<int> access(g.E);            // first bank counter of the access the edge takes part in
+  std::vector<int> bank(g.E), row(g.E), row_end(g.C, 0);
+  std::vector<uint8_t> count((size_t)groups * 32, 0);  // at most 32 variables share an access
+  for (int v = 0; v < g.V; ++v)
+    for (int q = g.var_ptr[v]; q < g.var_ptr[v + 1]; ++q)
+      access[g.var_edges[q]] = 32 * (v / 32 * K + (q - g.var_ptr[v]));
+  for (int e = 0; e < g.E; ++e) ++row_end[g.edge_chk[e]];
+  for (int c = 1; c < g.C; ++c) row_end[c] += row_end[c - 1];
+  for (int e = 0; e < g.E; ++e) {
+    const int c = g.edge_chk[e];
+    row[(c ? row_end[c - 1] : 0) + slot[e]] = e;
+    bank[e] = slot_index_host(slot[e], c, g.C, msg_type) * words / 4 % 32;
+    ++count[access[e] + bank[e]];
+  }
+  // a bank with n messages costs n^3 - n: an access waits for its fullest bank
+  int cost[34];
+  for (int n = 0; n < 34; ++n) cost[n] = n * (n * n - 1);
+  bool moved = true;
+  for (int sweep = 0; sweep < 3 && moved; ++sweep) {
+    moved = false;
+    for (int c = 0; c < g.C; ++c)
+      for (int i = c ? row_end[c - 1] : 0; i < row_end[c]; ++i)
+        for (int j = i + 1; j < row_end[c]; ++j) {
+          const int a = row[i], b = row[j], ba = bank[a], bb = bank[b];
+          if (ba == bb || access[a] == access[b]) continue;
+          uint8_t* ca = &count[access[a]];
+          uint8_t* cb = &count[access[b]];
+          if (cost[ca[ba] - 1] + cost[ca[bb] + 1] + cost[cb[ba] + 1] + cost[cb[bb] - 1] >=
+              cost[ca[ba]] + cost[ca[bb]] + cost[cb[ba]] + cost[cb[bb]])
+            continue;
+          --ca[ba], ++ca[bb], ++cb[ba], --cb[bb];
+          std::swap(slot[a], slot[b]);
+          std::swap(bank[a], bank[b]);
+          moved = true;
+        }
+  }
+  return slot;
+}
+
+// Entries per variable of the check-index table (DevGraph::var_chk): whole 8-byte loads.
+int chk_stride(int vslots) { return vslots <= 4 ? 4 : 8; }
 
 // Smallest supported owned-variable count covering V with G threads.
 int vpt_for(int V, int G) {
@@ -157,16 +227,19 @@ int vpt_for(int V, int G) {
 }
 
 // Default shape: the fewest owned variables per thread (from 3 up) whose group
-// still fits the register budget of that count (of the one- or two-shot
-// kernel, at one or two resident blocks per SM), so a shot's iteration is short.
-int default_group_threads(int C, int V, int nshots = 1, int vslots = 8, int minb = 1) {
+// still fits the register budget of that count, so a shot's iteration is short.
+int default_group_threads(int C, int V, int nshots = 1, int minb = 1) {
   for (int vpt : {3, 4, 6, 8, 12, 16}) {
     const int G = std::max(32, (V + vpt - 1) / vpt + 31) / 32 * 32;
-    const int max_threads = minb == 2 ? rbpk::max_slots_block_threads2(vpt)
-                                      : rbpk::max_slots_block_threads(vpt, nshots, vslots <= 3 ? 3 : 8);
-    if (G <= max_threads && (C + G - 1) / G <= 32 && vpt_for(V, G) <= vpt) return G;
+    if (G <= max_group_threads(vpt, nshots, minb) && (C + G - 1) / G <= 32 && vpt_for(V, G) <= vpt) return G;
   }
   return 256;  // configure reports why no shape fits
+}
+
+DevGraph device_graph(const rbp_decoder& d) {
+  const rbp_graph* g = d.g;
+  return DevGraph{g->C, g->V, g->E, g->slots, d.rows, g->vslots, g->chk_deg.p, g->chk_ptr.p,
+                  d.var_pos.p, d.var_chk.p, chk_stride(g->vslots)};
 }
 
 // Allow a kernel the device's opt-in shared memory minus its static shared
@@ -182,48 +255,12 @@ cudaError_t set_max_dynamic_smem(const void* kernel, size_t max_smem, size_t* st
                               (int)(max_smem - fa.sharedSizeBytes));
 }
 
-struct Launch {
-  KernelFn kernel;
-  int group_threads, groups, blocks;
-  int nshots;        // shots a group decodes at once
-  int slots_kernel;  // 1: relaybp_slots_kernel (one group per block, nshots shot regions)
-  int minb;          // resident blocks per SM the kernel is compiled for
-};
-
-// Block-per-group shape: one group of G threads per block with nshots shot regions
-// (relaybp_slots_kernel), compiled for minb (1 or 2) resident blocks per SM.
-int choose_slots_launch(int C, int V, int slots, int vslots, int rows, int msg_type, int G, int nshots, int minb,
-                        size_t max_smem, int sm_count, Launch* out, const std::string& w) {
-  const int vpt = vpt_for(V, G);
-  const int max_threads = minb == 2 ? rbpk::max_slots_block_threads2(vpt)
-                                    : rbpk::max_slots_block_threads(vpt, nshots, vslots <= 3 ? 3 : 8);
-  if (G > max_threads)
-    return fail(RBP_ERR_UNSUPPORTED, w + ": " + std::to_string(G) + " threads with " + std::to_string(vpt) +
-                                         " variables each exceed the register budget of " + std::to_string(nshots) +
-                                         "-shot groups" + (minb == 2 ? " at two blocks per SM" : ""));
-  KernelFn k = pick_slots_kernel(msg_type, slots, vslots, vpt, nshots, minb);
-  if (!k)
-    return fail(RBP_ERR_UNSUPPORTED,
-                w + (minb == 2 ? ": no two-blocks-per-SM kernel for this shape (one shot per group, check "
-                                 "degrees up to 16)"
-                               : ": no block-per-group kernel for this degree / shape (check degrees "
-                                 "above 16 run with several groups per block, one shot each)"));
-  const Layout L = make_layout(C, V, rows, msg_type, G, nshots == 1);
-  const size_t smem = (size_t)L.off_group0 + (size_t)nshots * L.group_bytes;
-  if (smem > max_smem)
-    return fail(RBP_ERR_UNSUPPORTED, w + ": " + std::to_string(nshots) + " shots' state (" +
-                                         std::to_string(nshots * L.group_bytes) + " B) does not fit in shared memory");
-  RBP_CUDA(set_max_dynamic_smem(reinterpret_cast<const void*>(k), max_smem));
-  int per_sm = 0;
-  RBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, G, smem));
-  if (per_sm < 1) return fail(RBP_ERR_UNSUPPORTED, w + ": launch shape has zero occupancy");
-  *out = Launch{k, G, 1, per_sm * sm_count, nshots, 1, minb};
-  return RBP_OK;
-}
-
 // Kernel and launch shape for G threads per group (groups_per_block 0: as many
-// as fit) decoding `nshots` shots at once (1 or 2); blocks_per_sm 2 selects the
-// block-per-group kernel compiled for two resident blocks per SM.
+// as fit).  blocks_per_sm 2 selects the kernel with one group per block compiled for
+// two resident blocks per SM.  nshots 2 (one group per block) asks for two shots per
+// group: checked against that shape's own limits and then run one shot after the
+// other (a kernel interleaving two shots in one group measured slower than one-shot
+// groups at every size of the benchmark code).
 int choose_launch(int C, int V, int slots, int vslots, int rows, int msg_type, int G, int groups_per_block,
                   size_t max_smem, int sm_count, Launch* out, const char* who, int nshots = 1,
                   int blocks_per_sm = 1) {
@@ -239,37 +276,42 @@ int choose_launch(int C, int V, int slots, int vslots, int rows, int msg_type, i
   if (blocks_per_sm == 2 && (nshots != 1 || groups_per_block != 1))
     return fail(RBP_ERR_UNSUPPORTED, w + ": two blocks per SM run the block-per-group kernel with one shot per "
                                          "group (groups_per_block 1, shots_per_group 1)");
-  // groups_per_block 1, or two shots per group: the block-per-group kernel
-  if (nshots == 2 || groups_per_block == 1) {
-    if (groups_per_block > 1)
-      return fail(RBP_ERR_UNSUPPORTED, w + ": two-shot groups run one group per block");
-    return choose_slots_launch(C, V, slots, vslots, rows, msg_type, G, nshots, blocks_per_sm, max_smem, sm_count,
-                               out, w);
-  }
-  const int max_threads = rbpk::max_block_threads(vpt);
+  const bool block_per_group = nshots == 2 || groups_per_block == 1;
+  if (nshots == 2 && groups_per_block > 1)
+    return fail(RBP_ERR_UNSUPPORTED, w + ": two-shot groups run one group per block");
+  const int max_threads = max_group_threads(vpt, nshots, blocks_per_sm);
   if (G > max_threads)
     return fail(RBP_ERR_UNSUPPORTED, w + ": " + std::to_string(G) + " threads with " + std::to_string(vpt) +
-                                         " variables each exceed the register budget");
-  KernelFn k = pick_kernel(msg_type, slots, vslots, vpt);
+                                         " variables each exceed the register budget" +
+                                         (blocks_per_sm == 2 ? " at two blocks per SM" : ""));
+  if (block_per_group && slots > 16)
+    return fail(RBP_ERR_UNSUPPORTED, w + ": no block-per-group kernel for this degree / shape (check degrees "
+                                         "above 16 run with several groups per block, one shot each)");
+  KernelFn k = blocks_per_sm == 2 ? pick2_kernel(msg_type, slots, vslots, vpt) : pick_kernel(msg_type, slots, vslots, vpt);
   if (!k) return fail(RBP_ERR_UNSUPPORTED, w + ": no kernel for this degree / shape");
-  const Layout L = make_layout(C, V, rows, msg_type, G);
-  const size_t block_fixed = (size_t)L.off_group0;
-  if (block_fixed + L.group_bytes > max_smem)
-    return fail(RBP_ERR_UNSUPPORTED,
-                w + ": one shot's state (" + std::to_string(L.group_bytes) + " B) does not fit in shared memory");
-  int max_groups = (int)((max_smem - block_fixed) / L.group_bytes);
-  max_groups = std::min(max_groups, max_threads / G);
-  if (G != 32) max_groups = std::min(max_groups, 15);  // named barriers 1..15
-  const int NG = groups_per_block > 0 ? groups_per_block : max_groups;
-  if (NG < 1 || NG > max_groups)
-    return fail(RBP_ERR_UNSUPPORTED,
-                w + ": groups_per_block must be in [1, " + std::to_string(max_groups) + "] for this shape");
+  const Layout bare = make_layout(C, V, rows, msg_type, G, vpt, false);
+  const size_t block_fixed = (size_t)bare.off_group0;
+  if (block_fixed + (size_t)nshots * bare.group_bytes > max_smem)
+    return fail(RBP_ERR_UNSUPPORTED, w + ": the state of " + std::to_string(nshots) + " shot(s) (" +
+                                         std::to_string(nshots * bare.group_bytes) +
+                                         " B) does not fit in shared memory");
+  int NG = 1;
+  if (!block_per_group) {
+    int max_groups = (int)((max_smem - block_fixed) / bare.group_bytes);
+    max_groups = std::min(max_groups, max_threads / G);
+    if (G != 32) max_groups = std::min(max_groups, 15);  // named barriers 1..15
+    NG = groups_per_block > 0 ? groups_per_block : max_groups;
+    if (NG < 1 || NG > max_groups)
+      return fail(RBP_ERR_UNSUPPORTED,
+                  w + ": groups_per_block must be in [1, " + std::to_string(max_groups) + "] for this shape");
+  }
+  const Layout L = fit_layout(C, V, rows, msg_type, G, vpt, NG, max_smem);
   RBP_CUDA(set_max_dynamic_smem(reinterpret_cast<const void*>(k), max_smem));
   const size_t smem = block_fixed + (size_t)NG * L.group_bytes;
   int per_sm = 0;
   RBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, G * NG, smem));
   if (per_sm < 1) return fail(RBP_ERR_UNSUPPORTED, w + ": launch shape has zero occupancy");
-  *out = Launch{k, G, NG, per_sm * sm_count, 1, 0, 1};
+  *out = Launch{k, G, NG, per_sm * sm_count, nshots, blocks_per_sm, L};
   return RBP_OK;
 }
 
@@ -305,11 +347,23 @@ int check_batch(const char* who, int64_t B, const rbp_batch* in, const rbp_outpu
   return RBP_OK;
 }
 
+// Whether a check's outputs could be non-finite, so that its rows need the masked form
+// (relaybp_rows.cuh): magnitudes are at most 1e30 before alpha and beta, and eight of
+// them must add up to a finite number.
+bool strict_rows(const rbp_params& p, const float* alpha, int n_alpha) {
+  if (p.use_beta && !(p.beta >= 0.0f)) return true;
+  for (int i = 0; p.use_alpha && i < n_alpha; ++i)
+    if (!(std::fabs(alpha[i]) <= 1e6f)) return true;
+  return false;
+}
+
 // Fill the kernel arguments and launch (memset of the work counter + kernel) on `st`.
-int launch_decode(const DevGraph& dgph, const rbp_params& p, const Layout& L, const Launch& lc, const float* llr,
-                  const float* gamma_legs, const float* alpha, int* queue, int64_t B,
-                  const rbp_batch* in, const rbp_outputs* out, cudaStream_t st, const char* who) {
+int launch_decode(const DevGraph& dgph, const rbp_params& p, const Launch& lc, const float* llr,
+                  const float* gamma_legs, const float* alpha, bool strict, int* queue, int64_t B, const rbp_batch* in, const rbp_outputs* out, cudaStream_t st, const char* who) {
+  const Layout& L = lc.L;
   DevArgs a{};
+  a.strict = strict;
+  a.keep_sums = L.sums;
   a.pre_iter = in->pre_iter;
   a.num_sets = p.num_sets;
   a.set_max_iter = p.set_max_iter;
@@ -336,7 +390,6 @@ int launch_decode(const DevGraph& dgph, const rbp_params& p, const Layout& L, co
   a.solved_gamma = in->solved_gamma;
   a.solved_legs = in->solved_legs;
   a.suspend_unsolved = in->suspend_unsolved;
-  a.parity_first = in->parity_first;
   a.init_post = in->init_posterior;
   a.errors = out->errors;
   a.errors_packed = out->errors_packed;
@@ -365,10 +418,9 @@ int launch_decode(const DevGraph& dgph, const rbp_params& p, const Layout& L, co
   a.g_first = L.g_first;
   a.g_red = L.g_red;
   a.g_s1 = L.g_s1;
-  const long long per_block = (long long)lc.groups * lc.nshots;  // shots a block decodes at once
-  const long long need_blocks = (B + per_block - 1) / per_block;
+  const long long need_blocks = (B + lc.groups - 1) / lc.groups;
   const int blocks = (int)std::min<long long>(lc.blocks, need_blocks);
-  const size_t smem = (size_t)L.off_group0 + (size_t)per_block * L.group_bytes;
+  const size_t smem = (size_t)L.off_group0 + (size_t)lc.groups * L.group_bytes;
   cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(int), st);
   if (e != cudaSuccess) return fail(RBP_ERR_CUDA, std::string(who) + ": cudaMemsetAsync: " + cudaGetErrorString(e));
   lc.kernel<<<blocks, lc.group_threads * lc.groups, smem, st>>>(dgph, a);
@@ -500,29 +552,15 @@ int rbp_decoder_configure_kind(rbp_decoder* d, int32_t kind, int32_t group_threa
     if (nshots != 1) return fail(RBP_ERR_ARGUMENT, "rbp_decoder_configure: groups_per_block -1 runs one shot per group");
     groups_per_block = 0;
   }
-  const bool block_per_group = nshots == 2 || groups_per_block == 1;
-  // default group size within the register budget of the kernel family that runs it
-  const int G = group_threads > 0 ? group_threads
-                                  : default_group_threads(g->C, g->V, nshots, block_per_group ? g->vslots : 8, minb);
+  // default group size within the register budget of the kernel that runs it
+  const int G = group_threads > 0 ? group_threads : default_group_threads(g->C, g->V, nshots, minb);
   DeviceGuard dg(g->device);
   Launch lc{};
   const int rc = choose_launch(g->C, g->V, g->slots, g->vslots, d->rows, d->p.msg_type, G, groups_per_block,
                                d->max_smem, d->sm_count, &lc, "rbp_decoder_configure", nshots, minb);
   if (rc != RBP_OK) return rc;
-  const Layout L = make_layout(g->C, g->V, d->rows, d->p.msg_type, G, lc.slots_kernel && lc.nshots == 1);
-  rbp_decoder::Shape sh;
-  sh.kernel = lc.kernel;
-  sh.vpt = vpt_for(g->V, G);
-  sh.group_threads = lc.group_threads;
-  sh.groups = lc.groups;
-  sh.blocks = lc.blocks;
-  sh.nshots = lc.nshots;
-  sh.slots_kernel = lc.slots_kernel;
-  sh.minb = lc.minb;
-  sh.group_bytes = L.group_bytes;
-  sh.block_bytes = L.off_group0;
-  if (kind != RBP_LAUNCH_LEGS) d->shape[0] = sh;
-  if (kind != RBP_LAUNCH_PRE) d->shape[1] = sh;
+  if (kind != RBP_LAUNCH_LEGS) d->shape[0] = lc;
+  if (kind != RBP_LAUNCH_PRE) d->shape[1] = lc;
   return RBP_OK;
 }
 
@@ -559,14 +597,19 @@ int rbp_decoder_create(const rbp_graph* g, const rbp_params* p, const float* llr
   }
   {
     std::vector<uint16_t> h_var_pos((size_t)g->vslots * g->V, rbpk::kNoSlot);
+    const int cs = chk_stride(g->vslots);
+    std::vector<uint16_t> h_var_chk((size_t)cs * g->V, rbpk::kNoSlot);
+    const std::vector<int> slot = conflict_free_slots(*g, p->msg_type);
     for (int v = 0; v < g->V; ++v)
       for (int k = g->var_ptr[v]; k < g->var_ptr[v + 1]; ++k) {
         const int e = g->var_edges[k];
         h_var_pos[(size_t)(k - g->var_ptr[v]) * g->V + v] =
-            (uint16_t)slot_index_host(g->edge_slot[e], g->edge_chk[e], g->C, p->msg_type);
+            (uint16_t)slot_index_host(slot[e], g->edge_chk[e], g->C, p->msg_type);
+        h_var_chk[(size_t)v * cs + (k - g->var_ptr[v])] = (uint16_t)g->edge_chk[e];
       }
     int rc0;
-    if ((rc0 = d->var_pos.upload(h_var_pos.data(), h_var_pos.size()))) {
+    if ((rc0 = d->var_pos.upload(h_var_pos.data(), h_var_pos.size())) ||
+        (rc0 = d->var_chk.upload(h_var_chk.data(), h_var_chk.size()))) {
       delete d;
       return rc0;
     }
@@ -575,6 +618,7 @@ int rbp_decoder_create(const rbp_graph* g, const rbp_params* p, const float* llr
   if (p->use_alpha) a_host.assign(alpha, alpha + n_alpha);
   else a_host.assign(1, 1.0f);
   d->n_alpha = (int)a_host.size();
+  d->strict = strict_rows(*p, a_host.data(), d->n_alpha);
   int zero = 0, rc;
   if ((rc = d->gamma_legs.upload(gamma_legs, (size_t)p->num_sets * g->V)) ||
       (rc = d->alpha.upload(a_host.data(), a_host.size())) || (rc = d->queue.upload(&zero, 1)) ||
@@ -615,8 +659,8 @@ int rbp_state_posterior_offset(const rbp_decoder* d, int64_t* offset) {
 int rbp_decoder_query(const rbp_decoder* d, int64_t* group_smem, int64_t* block_smem, int32_t* group_threads,
                       int32_t* groups_per_block, int32_t* blocks, int32_t* shots_per_group) {
   if (!d) return fail(RBP_ERR_ARGUMENT, "rbp_decoder_query: null decoder");
-  if (group_smem) *group_smem = d->shape[1].group_bytes;
-  if (block_smem) *block_smem = d->shape[1].block_bytes;
+  if (group_smem) *group_smem = d->shape[1].L.group_bytes;
+  if (block_smem) *block_smem = d->shape[1].L.off_group0;
   return rbp_decoder_query_kind(d, RBP_LAUNCH_LEGS, group_threads, groups_per_block, shots_per_group, nullptr,
                                 blocks);
 }
@@ -626,7 +670,7 @@ int rbp_decoder_query_kind(const rbp_decoder* d, int32_t kind, int32_t* group_th
   if (!d) return fail(RBP_ERR_ARGUMENT, "rbp_decoder_query: null decoder");
   if (kind != RBP_LAUNCH_PRE && kind != RBP_LAUNCH_LEGS)
     return fail(RBP_ERR_ARGUMENT, "rbp_decoder_query: kind must be RBP_LAUNCH_PRE or RBP_LAUNCH_LEGS");
-  const rbp_decoder::Shape& sh = d->shape[kind == RBP_LAUNCH_PRE ? 0 : 1];
+  const Launch& sh = d->shape[kind == RBP_LAUNCH_PRE ? 0 : 1];
   if (group_threads) *group_threads = sh.group_threads;
   if (groups_per_block) *groups_per_block = sh.groups;
   if (shots_per_group) *shots_per_group = sh.nshots;
@@ -643,11 +687,8 @@ int rbp_decode(rbp_decoder* d, int64_t B, const rbp_batch* in, const rbp_outputs
   DeviceGuard dg(g->device);
   if (!dg.ok) return fail(RBP_ERR_CUDA, "rbp_decode: cannot select the CUDA device");
   // a launch that skips the relay legs runs at most pre_iter iterations per shot
-  const rbp_decoder::Shape& sh = d->shape[in->skip_relay_legs ? 0 : 1];
-  const Layout L = make_layout(g->C, g->V, d->rows, d->p.msg_type, sh.group_threads, sh.slots_kernel && sh.nshots == 1);
-  const DevGraph dgph{g->C, g->V, g->E, g->slots, d->rows, g->vslots, g->chk_deg.p, g->chk_ptr.p, d->var_pos.p};
-  const Launch lc{sh.kernel, sh.group_threads, sh.groups, sh.blocks, sh.nshots, sh.slots_kernel, sh.minb};
-  return launch_decode(dgph, d->p, L, lc, d->llr.p, d->gamma_legs.p, d->alpha.p, d->queue.p, B, in,
+  const Launch& sh = d->shape[in->skip_relay_legs ? 0 : 1];
+  return launch_decode(device_graph(*d), d->p, sh, d->llr.p, d->gamma_legs.p, d->alpha.p, d->strict, d->queue.p, B, in,
                        out, reinterpret_cast<cudaStream_t>(stream), "rbp_decode");
 }
 
@@ -660,6 +701,7 @@ struct rbp_mixed {
   int device = 0;
   const rbp_decoder* dec[rbpk::kMaxMixedCodes] = {};
   int G[rbpk::kMaxMixedCodes] = {}, NG[rbpk::kMaxMixedCodes] = {};
+  Layout L[rbpk::kMaxMixedCodes] = {};
   rbpk::MixedKernelFn kernel = nullptr;
   int vpt = 0;                 // owned variables per thread of the instantiation
   int block_threads = 0, blocks = 0;
@@ -677,6 +719,8 @@ struct rbp_mixed {
 
 namespace {
 
+constexpr size_t kMixedStatic = 64;  // shared memory left for the mixed kernel's own variables
+
 // Kernel arguments of one mixed launch.
 int mixed_args(rbp_mixed* m, const int64_t* B, const rbp_batch* ins, const rbp_outputs* outs, rbpk::MixedArgs* ma) {
   std::memset(ma, 0, sizeof(*ma));
@@ -687,13 +731,14 @@ int mixed_args(rbp_mixed* m, const int64_t* B, const rbp_batch* ins, const rbp_o
     const rbp_graph* g = d->g;
     int rc = check_batch("rbp_mixed_decode", B[i], &ins[i], &outs[i], d->p, d->n_alpha);
     if (rc != RBP_OK) return rc;
-    const Layout L = make_layout(g->C, g->V, d->rows, d->p.msg_type, m->G[i]);
-    ma->code[i].g = DevGraph{g->C, g->V, g->E, g->slots, d->rows, g->vslots, g->chk_deg.p, g->chk_ptr.p,
-                             d->var_pos.p};
+    const Layout& L = m->L[i];
+    ma->code[i].g = device_graph(*d);
     DevArgs& a = ma->code[i].a;
+    a.keep_sums = L.sums;
     const rbp_params& p = d->p;
     const rbp_batch* in = &ins[i];
     const rbp_outputs* out = &outs[i];
+    a.strict = d->strict;
     a.pre_iter = in->pre_iter;
     a.num_sets = p.num_sets;
     a.set_max_iter = p.set_max_iter;
@@ -720,8 +765,7 @@ int mixed_args(rbp_mixed* m, const int64_t* B, const rbp_batch* ins, const rbp_o
     a.solved_gamma = in->solved_gamma;
     a.solved_legs = in->solved_legs;
     a.suspend_unsolved = in->suspend_unsolved;
-    a.parity_first = in->parity_first;
-    a.init_post = in->init_posterior;
+      a.init_post = in->init_posterior;
     a.errors = out->errors;
     a.errors_packed = out->errors_packed;
     a.weights = out->weights;
@@ -739,7 +783,7 @@ int mixed_args(rbp_mixed* m, const int64_t* B, const rbp_batch* ins, const rbp_o
     a.groups = m->NG[i];
     a.off_chk_deg = L.off_chk_deg;
     a.off_llr = L.off_llr;
-    a.off_first = L.off_first;
+      a.off_first = L.off_first;
     a.first_table = 1;
     a.off_group0 = L.off_group0;
     a.group_bytes = L.group_bytes;
@@ -824,12 +868,14 @@ int rbp_mixed_create(const rbp_decoder* const* decoders, int32_t n, rbp_mixed** 
         if ((T / k) % 32) continue;
         const int Gc = T / k;
         if (vpt_for(g->V, Gc) < 0 || vpt_for(g->V, Gc) > vpt || (g->C + Gc - 1) / Gc > 32) continue;
-        const Layout L = make_layout(g->C, g->V, d->rows, d->p.msg_type, Gc);
+        const Layout bare = make_layout(g->C, g->V, d->rows, d->p.msg_type, Gc, vpt, false);
         int ng = std::min(k, Gc == 32 ? k : 15);
-        while (ng >= 1 && (size_t)L.off_group0 + (size_t)ng * L.group_bytes > d->max_smem) --ng;
+        while (ng >= 1 && (size_t)bare.off_group0 + (size_t)ng * bare.group_bytes > d->max_smem) --ng;
         if (ng < 1) continue;
         best_G = Gc;
         best_NG = ng;
+        const Layout L = fit_layout(g->C, g->V, d->rows, d->p.msg_type, Gc, vpt, ng, d->max_smem - kMixedStatic);
+        m->L[i] = L;
         smem = std::max(smem, (size_t)L.off_group0 + (size_t)ng * L.group_bytes);
         break;
       }
@@ -938,6 +984,7 @@ int rbp_mixed_configure(rbp_mixed* m, const int32_t* group_threads) {
   if (!m || !group_threads) return fail(RBP_ERR_ARGUMENT, "rbp_mixed_configure: null argument");
   const int T = m->block_threads;
   int G[rbpk::kMaxMixedCodes], NG[rbpk::kMaxMixedCodes];
+  Layout Ls[rbpk::kMaxMixedCodes];
   size_t smem = 0;
   for (int i = 0; i < m->n; ++i) {
     const rbp_decoder* d = m->dec[i];
@@ -952,11 +999,13 @@ int rbp_mixed_configure(rbp_mixed* m, const int32_t* group_threads) {
       return fail(RBP_ERR_UNSUPPORTED, "rbp_mixed_configure: code " + std::to_string(i) + ": " +
                                            std::to_string(Gi) + " threads own more than " + std::to_string(m->vpt) +
                                            " variables or 32 checks each");
-    const Layout L = make_layout(g->C, g->V, d->rows, d->p.msg_type, Gi);
+    const Layout bare = make_layout(g->C, g->V, d->rows, d->p.msg_type, Gi, m->vpt, false);
     int ng = std::min(T / Gi, Gi == 32 ? T / Gi : 15);
-    while (ng >= 1 && (size_t)L.off_group0 + (size_t)ng * L.group_bytes > d->max_smem) --ng;
+    while (ng >= 1 && (size_t)bare.off_group0 + (size_t)ng * bare.group_bytes > d->max_smem) --ng;
     if (ng < 1)
       return fail(RBP_ERR_UNSUPPORTED, "rbp_mixed_configure: code " + std::to_string(i) + ": no group fits");
+    const Layout L = fit_layout(g->C, g->V, d->rows, d->p.msg_type, Gi, m->vpt, ng, d->max_smem - kMixedStatic);
+    Ls[i] = L;
     G[i] = Gi;
     NG[i] = ng;
     smem = std::max(smem, (size_t)L.off_group0 + (size_t)ng * L.group_bytes);
@@ -968,6 +1017,7 @@ int rbp_mixed_configure(rbp_mixed* m, const int32_t* group_threads) {
   for (int i = 0; i < m->n; ++i) {
     m->G[i] = G[i];
     m->NG[i] = NG[i];
+    m->L[i] = Ls[i];
   }
   m->smem = smem;
   m->blocks = per_sm * m->dec[0]->sm_count;
@@ -1015,11 +1065,13 @@ int rbp_decode_static(int32_t C, int32_t V, int32_t E, const int32_t* chk_ptr, c
   const int rows = layout_rows(slots, p->msg_type);
   if ((long long)rows * C >= 65535)
     return fail(RBP_ERR_UNSUPPORTED, std::string(who) + ": message layout exceeds 65535 slots");
-  // scratch layout: [counter | chk_deg u8 | chk_ptr i32 | var_pos u16]
+  // scratch layout: [counter | chk_deg u8 | chk_ptr i32 | var_pos u16 | var_chk u16]
   const size_t off_deg = 256;
   const size_t off_ptr = (off_deg + (size_t)C + 15) / 16 * 16;
   const size_t off_pos = (off_ptr + 4 * ((size_t)C + 1) + 15) / 16 * 16;
-  const size_t need = off_pos + 2 * (size_t)vslots * V;
+  const int cs = chk_stride(vslots);
+  const size_t off_chk = (off_pos + 2 * (size_t)vslots * V + 15) / 16 * 16;
+  const size_t need = off_chk + 2 * (size_t)cs * V;
   if (need > (size_t)RBP_STATIC_SCRATCH_BYTES)
     return fail(RBP_ERR_UNSUPPORTED, std::string(who) + ": graph tables need " + std::to_string(need) +
                                          " bytes of scratch; the static scratch holds " +
@@ -1088,17 +1140,30 @@ int rbp_decode_static(int32_t C, int32_t V, int32_t E, const int32_t* chk_ptr, c
     }
   }
   if ((rc = flush())) return rc;
+  at = off_chk;
+  for (int v = 0; v < V; ++v) {
+    for (int k = 0; k < cs; ++k) {
+      uint16_t c = rbpk::kNoSlot;
+      if (var_ptr[v] + k < var_ptr[v + 1])
+        c = (uint16_t)(std::upper_bound(chk_ptr, chk_ptr + C + 1, var_edges[var_ptr[v] + k]) - chk_ptr - 1);
+      std::memcpy(stage + fill, &c, 2);
+      fill += 2;
+      if (fill == sizeof(stage) && (rc = flush())) return rc;
+    }
+  }
+  if ((rc = flush())) return rc;
 
   int G = default_group_threads(C, V), max_smem = 0, sms = 0;
   RBP_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   RBP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   Launch lc{};
   if ((rc = choose_launch(C, V, slots, vslots, rows, p->msg_type, G, 0, (size_t)max_smem, sms, &lc, who))) return rc;
-  const Layout L = make_layout(C, V, rows, p->msg_type, G);
   const DevGraph dgph{C, V, E, slots, rows, vslots, scratch + off_deg, reinterpret_cast<const int*>(scratch + off_ptr),
-                      reinterpret_cast<const uint16_t*>(scratch + off_pos)};
-  return launch_decode(dgph, *p, L, lc, llr, gamma_legs, alpha, reinterpret_cast<int*>(scratch), B, in, out,
-                       st, who);
+                      reinterpret_cast<const uint16_t*>(scratch + off_pos),
+                      reinterpret_cast<const uint16_t*>(scratch + off_chk), cs};
+  return launch_decode(dgph, *p, lc, llr, gamma_legs, alpha,
+                       p->use_alpha || strict_rows(*p, nullptr, 0),  // the alpha table is on the device
+                       reinterpret_cast<int*>(scratch), B, in, out, st, who);
 }
 
 }  // extern "C"
