@@ -4,9 +4,13 @@
 // observables of true and decoded errors (O e, O e_hat).  The reference does
 // both on the host with scipy (src/pelagos/adapter.py:545-560, 601-613, 679).
 //
-// One thread block per shot at a time: the shot's x row (N bytes) is staged in
-// shared memory once and every row of the matrix is evaluated against it, so a
-// shot's bytes cross DRAM once however many rows the matrix has.
+// Shots are bit-sliced: a block takes up to 32 shots, turns their columns into
+// words (bit b of word j: column j of shot b) in shared memory, and a row is the
+// XOR of its columns' words, so one shared-memory read serves 32 shots.
+// Measured with 65,536 shots: the 936 x 2,592 check matrix (231 MB in and out)
+// 611 -> 83 us, the 12 observables of long rows 450 -> 42 us, against a
+// shot's bytes staged and gathered one by one; reading x once at the copy
+// bandwidth takes 26 us.
 
 #include "relaybp.h"
 #include "relaybp_host.h"
@@ -21,24 +25,113 @@ namespace {
 using rbph::fail;
 
 constexpr int GF2_THREADS = 256;
+constexpr int GF2_SHOTS = 32;  // shots per tile: the bits of a word
 
-// Block b handles shot b (grid-stride): stage x[b, :] in shared memory, then
-// each thread evaluates rows r = threadIdx.x, threadIdx.x + blockDim.x, ...
-__global__ void __launch_bounds__(GF2_THREADS) gf2_rows_kernel(const uint8_t* x, long long B, int N,
+// Bit r of lane c's word becomes bit c of lane r's (5 exchanges of half blocks).
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, int lane) {
+  uint32_t m = 0x0000ffffu;
+#pragma unroll
+  for (int j = 16; j > 0; j >>= 1) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? (x & ~m) | ((y >> j) & m) : (x & m) | ((y & m) << j);
+    m ^= m << (j >> 1);
+  }
+  return x;
+}
+
+// Low bits of a word's four bytes as a nibble, and back.
+__device__ __forceinline__ uint32_t pack4(uint32_t v) { return ((v & 0x01010101u) * 0x01020408u) >> 24 & 0xfu; }
+__device__ __forceinline__ uint32_t spread4(uint32_t n) { return ((n & 0xfu) * 0x00204081u) & 0x01010101u; }
+
+// Columns j0 .. j0+31 of one shot as a word (columns past N: 0).  VEC: bytes per load
+// (16 or 4 where every row's start is aligned to that, else 1).
+template <int VEC>
+__device__ __forceinline__ uint32_t load_columns(const uint8_t* row, int j0, int N) {
+  uint32_t w = 0u;
+  if (VEC == 16 && j0 + 32 <= N) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(row + j0 + 16 * h));
+      w |= (pack4(u.x) | pack4(u.y) << 4 | pack4(u.z) << 8 | pack4(u.w) << 12) << (16 * h);
+    }
+  } else if (VEC >= 4 && j0 + 32 <= N) {
+#pragma unroll
+    for (int h = 0; h < 8; ++h) w |= pack4(__ldg(reinterpret_cast<const uint32_t*>(row + j0 + 4 * h))) << (4 * h);
+  } else {
+    for (int h = 0; h < 32 && j0 + h < N; ++h) w |= (uint32_t)(row[j0 + h] & 1u) << h;
+  }
+  return w;
+}
+
+// Bits of w to n (<= 32) bytes.  VEC: 8, 4 or 1, as for load_columns.
+template <int VEC>
+__device__ __forceinline__ void store_bytes(uint8_t* p, uint32_t w, int n) {
+  if (VEC == 8 && n == 32) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      *reinterpret_cast<uint2*>(p + 8 * h) = make_uint2(spread4(w >> (8 * h)), spread4(w >> (8 * h + 4)));
+  } else if (VEC >= 4 && n == 32) {
+#pragma unroll
+    for (int h = 0; h < 8; ++h) *reinterpret_cast<uint32_t*>(p + 4 * h) = spread4(w >> (4 * h));
+  } else {
+    for (int h = 0; h < n; ++h) p[h] = (uint8_t)((w >> h) & 1u);
+  }
+}
+
+// Tiles of `tile` (1..32) shots, grid-stride.  A warp turns 32 columns of the tile's shots
+// (lane b: shot b) into 32 column words at a time; then a thread evaluates a row, or with
+// few rows (WARP_ROWS; they tend to be long: logical operators) a warp does.
+template <int IN, int OUT, bool WARP_ROWS>
+__global__ void __launch_bounds__(GF2_THREADS) gf2_rows_kernel(const uint8_t* x, long long B, int tile, int N,
                                                              const int* row_ptr, const int* cols, int R,
                                                              uint8_t* out) {
-  extern __shared__ __align__(16) uint8_t sx[];
-  for (long long b = blockIdx.x; b < B; b += gridDim.x) {
-    const uint8_t* xr = x + b * (long long)N;
-    __syncthreads();  // the previous shot's rows are done with sx
-    for (int j = threadIdx.x; j < N; j += blockDim.x) sx[j] = xr[j];
-    __syncthreads();
-    for (int r = threadIdx.x; r < R; r += blockDim.x) {
-      uint32_t p = 0;
-      for (int k = row_ptr[r]; k < row_ptr[r + 1]; ++k) p ^= sx[cols[k]];
-      out[b * (long long)R + r] = (uint8_t)(p & 1u);
+  extern __shared__ uint32_t word[];  // [N rounded up to 32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = GF2_THREADS / 32;
+  for (long long b0 = blockIdx.x * (long long)tile; b0 < B; b0 += gridDim.x * (long long)tile) {
+    const int nb = (int)min((long long)tile, B - b0);
+    const uint8_t* row = x + (b0 + min(lane, nb - 1)) * N;
+    for (int j0 = warp * 32; j0 < N; j0 += nwarps * 32) {
+      const uint32_t w = lane < nb ? load_columns<IN>(row, j0, N) : 0u;
+      word[j0 + lane] = transpose32(w, lane);
     }
+    __syncthreads();
+    if constexpr (WARP_ROWS) {
+      for (int r = warp; r < R; r += nwarps) {
+        uint32_t p = 0u;
+        for (int k = row_ptr[r] + lane; k < row_ptr[r + 1]; k += 32) p ^= word[cols[k]];
+        p = __reduce_xor_sync(0xffffffffu, p);
+        if (lane < nb) out[(b0 + lane) * R + r] = (uint8_t)((p >> lane) & 1u);
+      }
+    } else {
+      for (int r0 = warp * 32; r0 < R; r0 += nwarps * 32) {
+        uint32_t p = 0u;
+        if (r0 + lane < R)
+          for (int k = row_ptr[r0 + lane]; k < row_ptr[r0 + lane + 1]; ++k) p ^= word[cols[k]];
+        p = transpose32(p, lane);
+        if (lane < nb) store_bytes<OUT>(out + (b0 + lane) * R + r0, p, min(32, R - r0));
+      }
+    }
+    __syncthreads();  // the next tile overwrites the words
   }
+}
+
+template <int IN, int OUT>
+int launch_rows(const uint8_t* x, long long B, int N, const int* row_ptr, const int* cols, int R, uint8_t* out,
+                cudaStream_t st) {
+  const size_t smem = (size_t)((N + 31) / 32 * 32) * sizeof(uint32_t);
+  // fewer than 64 rows do not fill the block's threads
+  auto kernel = R < 64 ? gf2_rows_kernel<IN, OUT, true> : gf2_rows_kernel<IN, OUT, false>;
+  if (smem > 48 * 1024)
+    RBP_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem));
+  // whole words of shots once every SM has work for its resident blocks; small batches are
+  // spread over the SMs instead
+  const long long spread = 148LL * 4;
+  const int tile = (int)std::min<long long>(GF2_SHOTS, std::max<long long>(1, (B + spread - 1) / spread));
+  const int blocks = (int)std::min<long long>((B + tile - 1) / tile, 148LL * 8);
+  kernel<<<blocks, GF2_THREADS, smem, st>>>(x, B, tile, N, row_ptr, cols, R, out);
+  RBP_CUDA(cudaGetLastError());
+  return RBP_OK;
 }
 
 }  // namespace
@@ -49,9 +142,14 @@ extern "C" int rbp_gf2_matvec(const uint8_t* x, int64_t B, int32_t N, const int3
   if (B == 0 || R == 0) return RBP_OK;
   if (!x || !row_ptr || !out || (!cols && N > 0)) return fail(RBP_ERR_ARGUMENT, "rbp_gf2_matvec: null buffer");
   if (N > 48 * 1024) return fail(RBP_ERR_UNSUPPORTED, "rbp_gf2_matvec: rows longer than 49,152 columns");
-  const int blocks = (int)std::min<long long>(B, 148LL * 8);
-  gf2_rows_kernel<<<blocks, GF2_THREADS, (size_t)std::max(N, 1), static_cast<cudaStream_t>(stream)>>>(
-      x, B, N, row_ptr, cols, R, out);
-  RBP_CUDA(cudaGetLastError());
-  return RBP_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const uintptr_t in = reinterpret_cast<uintptr_t>(x) | (uintptr_t)N, o = reinterpret_cast<uintptr_t>(out) | (uintptr_t)R;
+  const int iv = in % 16 == 0 ? 16 : (in % 4 == 0 ? 4 : 1), ov = o % 8 == 0 ? 8 : (o % 4 == 0 ? 4 : 1);
+  if (iv == 16 && ov == 8) return launch_rows<16, 8>(x, B, N, row_ptr, cols, R, out, st);
+  if (iv == 16 && ov == 4) return launch_rows<16, 4>(x, B, N, row_ptr, cols, R, out, st);
+  if (iv == 16) return launch_rows<16, 1>(x, B, N, row_ptr, cols, R, out, st);
+  if (iv == 4 && ov >= 4) return launch_rows<4, 4>(x, B, N, row_ptr, cols, R, out, st);
+  if (iv == 4) return launch_rows<4, 1>(x, B, N, row_ptr, cols, R, out, st);
+  return ov >= 4 ? launch_rows<1, 4>(x, B, N, row_ptr, cols, R, out, st)
+                 : launch_rows<1, 1>(x, B, N, row_ptr, cols, R, out, st);
 }
