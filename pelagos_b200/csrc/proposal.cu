@@ -775,6 +775,327 @@ __global__ void __launch_bounds__(PROPOSE_THREADS, 1) net_propose_kernel(NetGrap
   }
 }
 
+// ------------------------------------------------------------------ fused inference, low degrees
+//
+// The same network for graphs with at most 8 edges per check and 4 per variable (and
+// V <= 3072, C <= 1024): every value is computed by the same operations in the same order,
+// so outputs equal net_propose_kernel's bit for bit.  A shot there took 110 K cycles, 63 K
+// of them in the two message sums: one thread walked a row's edges through dependent
+// loads of bounds, indices and 16-byte rows, half of each 32-byte row's banks unused, and
+// every pass ran once per half of the channels.  Here
+//   * index rows are padded (8 checks' or 4 variables' indices in one load), absent edges
+//     pointing at a zero row (sums) or a zero gate (aggregation), so a row's loads are
+//     independent;
+//   * messages and sums lie as two arrays of 16-byte half rows: consecutive rows cover
+//     every bank;
+//   * a layer's aggregate overwrites the layer's messages in place (a check reads only its
+//     own message row), which makes room for the sums of all 16 channels at once;
+//   * the tanh feature stays in its owner's registers after the check inputs are formed;
+//   * unsat / deg comes from a table of the quotients;
+//   * the next shot's posterior and syndrome are loaded while this one is evaluated;
+//   * a check's edge types are packed into one word per shot.
+// Measured on the 936 x 2,592 graph: 16,384 shots 6.53 -> 3.55 ms.  Of a shot's 58 K cycles
+// the aggregations take 21 K (issue, ALU and shared-memory work within 25 % of each other),
+// the tile passes (mma.sync chains of 16 checks) 18 K, the sums 9 K, the rest 10 K.
+
+constexpr int FP_DC = 8, FP_DV = 4, FP_KV = 6, FP_KC = 2;  // index rows; variables and checks per thread
+constexpr int FP_LUT = (FP_DV + 1) * (FP_DV + 1);
+
+struct FastArgs {
+  const uint16_t* chk_idx;  // [C][8] variable of each edge, V beyond the degree
+  const uint16_t* var_idx;  // [V][4] check of each edge, C beyond the degree
+  int off_fr, off_gate, off_bias, off_lut, off_ci, off_vi, off_x, off_a1, off_a2, off_n, off_tu, off_ct, off_syn;
+};
+
+// Rows r0, r0+8 of an array of half rows ([2][C + 1][8] bf16) as an A fragment (zero past C).
+__device__ __forceinline__ void load_a_halves(const bf16* s, int r0, int tq, int C, uint32_t (&a)[4]) {
+  const int r1 = r0 + 8;
+  const bf16* h1 = s + (C + 1) * 8;
+  a[0] = r0 < C ? *reinterpret_cast<const uint32_t*>(s + r0 * 8 + 2 * tq) : 0u;
+  a[1] = r1 < C ? *reinterpret_cast<const uint32_t*>(s + r1 * 8 + 2 * tq) : 0u;
+  a[2] = r0 < C ? *reinterpret_cast<const uint32_t*>(h1 + r0 * 8 + 2 * tq) : 0u;
+  a[3] = r1 < C ? *reinterpret_cast<const uint32_t*>(h1 + r1 * 8 + 2 * tq) : 0u;
+}
+
+__device__ __forceinline__ void tile_message_halves(const uint32_t* fr, int fw, const uint32_t (&ga)[4][4], int r0,
+                                                    int lane, int tq, int C, bf16* s_m) {
+  float mc[2][4];
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt) {
+    mc[nt][0] = mc[nt][1] = mc[nt][2] = mc[nt][3] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const uint32_t* f = fr + fw + (nt * 8 + kk * 2) * 32 + lane;
+      mma_bf16(mc[nt], ga[kk], f[0], f[32]);
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < 2; ++nt) {
+    bf16* h = s_m + nt * (C + 1) * 8;
+    if (r0 < C) *reinterpret_cast<uint32_t*>(h + r0 * 8 + 2 * tq) = pack_bf16(mc[nt][0], mc[nt][1]);
+    if (r0 + 8 < C) *reinterpret_cast<uint32_t*>(h + (r0 + 8) * 8 + 2 * tq) = pack_bf16(mc[nt][2], mc[nt][3]);
+  }
+}
+
+// acc <- relu(acc) + b + a^ U^T, a^ from half rows, b the layer's 64 biases
+__device__ __forceinline__ void tile_update_halves(const uint32_t* fr, int fu, const bf16* bias, const bf16* s_a, int r0,
+                                                   int lane, int tq, int C, float (&acc)[8][4]) {
+  uint32_t a[4];
+  load_a_halves(s_a, r0, tq, C, a);
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    const float2 bb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(bias + nt * 8 + 2 * tq));
+    acc[nt][0] = fmaxf(acc[nt][0], 0.f) + bb.x;
+    acc[nt][1] = fmaxf(acc[nt][1], 0.f) + bb.y;
+    acc[nt][2] = fmaxf(acc[nt][2], 0.f) + bb.x;
+    acc[nt][3] = fmaxf(acc[nt][3], 0.f) + bb.y;
+    const uint32_t* f = fr + fu + nt * 64 + lane;
+    mma_bf16(acc[nt], a, f[0], f[32]);
+  }
+}
+
+// DV: variable degree bound (3 or 4).
+template <int DV>
+__global__ void __launch_bounds__(PROPOSE_THREADS, 1) net_propose_fast_kernel(NetGraph g, ProposeArgs pa, FastArgs fa) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint32_t* fr = reinterpret_cast<uint32_t*>(smem + fa.off_fr);
+  bf16* s_gate = reinterpret_cast<bf16*>(smem + fa.off_gate);  // [2][5][16], row 4 zero
+  bf16* s_bias = reinterpret_cast<bf16*>(smem + fa.off_bias);  // [2][64]
+  float* s_lut = reinterpret_cast<float*>(smem + fa.off_lut);  // [deg][unsat] quotients
+  const uint16_t* s_ci = reinterpret_cast<const uint16_t*>(smem + fa.off_ci);
+  const uint16_t* s_vi = reinterpret_cast<const uint16_t*>(smem + fa.off_vi);
+  bf16* s_x = reinterpret_cast<bf16*>(smem + fa.off_x);    // [C][8]
+  bf16* s_a1 = reinterpret_cast<bf16*>(smem + fa.off_a1);  // layer 1: messages, then aggregates
+  bf16* s_a2 = reinterpret_cast<bf16*>(smem + fa.off_a2);  // layer 2
+  bf16* s_n = reinterpret_cast<bf16*>(smem + fa.off_n);    // [2][V + 1][8]
+  float* s_th = reinterpret_cast<float*>(smem + fa.off_n);  // [V + 1] until the check inputs are formed
+  float* s_o = reinterpret_cast<float*>(smem + fa.off_n);   // [C + 1] after the last aggregation
+  uint8_t* s_tu = smem + fa.off_tu;                         // [V + 1] type | (deg * 5 + unsat) << 3
+  uint32_t* s_ct = reinterpret_cast<uint32_t*>(smem + fa.off_ct);  // [C] types of a check's edges, 3 bits each
+  uint8_t* s_syn = smem + fa.off_syn;                       // [C + 1]
+  const int C = g.C, V = g.V;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = PROPOSE_THREADS >> 5;
+  const int gq = lane >> 2, tq = lane & 3;
+  const int ntiles = (C + 15) >> 4;
+
+  for (int i = tid; i < FR_WORDS; i += PROPOSE_THREADS) fr[i] = fragment_word(pa.theta, i);
+  for (int i = tid; i < 2 * 5 * ND; i += PROPOSE_THREADS) {
+    const int layer = i / (5 * ND), t = i / ND % 5;
+    s_gate[i] = t < NTY ? pa.theta[(layer ? P_G2 : P_G1) + t * ND + i % ND] : __float2bfloat16_rn(0.f);
+  }
+  for (int i = tid; i < 2 * NH; i += PROPOSE_THREADS) s_bias[i] = pa.theta[(i < NH ? P_B1 : P_B2) + i % NH];
+  for (int i = tid; i < FP_LUT; i += PROPOSE_THREADS)
+    s_lut[i] = (float)(i % (FP_DV + 1)) / (float)max(i / (FP_DV + 1), 1);
+  for (int i = tid; i < C; i += PROPOSE_THREADS)
+    reinterpret_cast<uint4*>(smem + fa.off_ci)[i] = __ldg(reinterpret_cast<const uint4*>(fa.chk_idx) + i);
+  for (int i = tid; i < V; i += PROPOSE_THREADS)
+    reinterpret_cast<uint2*>(smem + fa.off_vi)[i] = __ldg(reinterpret_cast<const uint2*>(fa.var_idx) + i);
+  if (tid < 4) {  // the zero rows absent edges point at
+    bf16* z = (tid & 1 ? s_a2 : s_a1) + (tid >> 1) * (C + 1) * 8 + C * 8;
+    *reinterpret_cast<uint4*>(z) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (tid == 0) {
+    s_syn[C] = 0;
+    s_tu[V] = 4;  // the zero gate
+  }
+  const float oz0 = ldw(pa.theta, P_OZ), oz1 = ldw(pa.theta, P_OZ + 1), oz2 = ldw(pa.theta, P_OZ + 2),
+              oz3 = ldw(pa.theta, P_OZ + 3), ob = ldw(pa.theta, P_OB);
+
+  const long long n_items = pa.shot_list && pa.list_count ? (long long)min(max(*pa.list_count, 0), (int)pa.B) : pa.B;
+  auto shot_of = [&](long long item) -> long long {
+    if (item >= n_items) return -1;
+    const long long b = pa.shot_list ? (long long)pa.shot_list[item] : item;
+    return b < pa.B ? b : -1;
+  };
+  float nx[FP_KV] = {};      // the next shot's posterior and syndrome (this thread's variables and checks)
+  uint32_t ny[FP_KC] = {};
+  auto fetch = [&](long long b) {
+#pragma unroll
+    for (int k = 0; k < FP_KV; ++k) {
+      const int v = tid + k * PROPOSE_THREADS;
+      if (v < V) nx[k] = __ldg(pa.post + b * pa.post_stride + v);
+    }
+#pragma unroll
+    for (int k = 0; k < FP_KC; ++k) {
+      const int c = tid + k * PROPOSE_THREADS;
+      if (c < C) ny[k] = __ldg(pa.syn + b * C + c) & 1u;
+    }
+  };
+  long long item = blockIdx.x, b = shot_of(item);
+  if (b >= 0) fetch(b);
+  for (; item < n_items; item += gridDim.x) {
+    const long long next = shot_of(item + gridDim.x);
+    if (b < 0) {  // block-uniform: no barrier is skipped by part of the block
+      b = next;
+      if (b >= 0) fetch(b);
+      continue;
+    }
+    float th[FP_KV];
+#pragma unroll
+    for (int k = 0; k < FP_KC; ++k) {
+      const int c = tid + k * PROPOSE_THREADS;
+      if (c < C) s_syn[c] = (uint8_t)ny[k];
+    }
+    __syncthreads();
+    // variable features
+#pragma unroll
+    for (int k = 0; k < FP_KV; ++k) {
+      const int v = tid + k * PROPOSE_THREADS;
+      if (v < V) {
+        const float pc = fminf(fmaxf(nx[k], -1e4f), 1e4f);
+        const uint2 u = reinterpret_cast<const uint2*>(s_vi)[v];
+        const int c[4] = {(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y & 0xffffu), (int)(u.y >> 16)};
+        int cnt = 0, deg = 0;
+#pragma unroll
+        for (int j = 0; j < DV; ++j) {
+          cnt += s_syn[c[j]];
+          deg += c[j] < C;
+        }
+        th[k] = tanhf(pc * 0.0625f);
+        s_th[v] = th[k];
+        s_tu[v] = (uint8_t)((pc <= 0.f ? 2 : 0) + (fabsf(pc) < 8.f ? 1 : 0) + ((deg * (FP_DV + 1) + cnt) << 3));
+      }
+    }
+    if (tid == 0) s_th[V] = 0.f;
+    __syncthreads();
+    if (next >= 0) fetch(next);
+    // check inputs x^ = (s, mean tanh, mean hard, mean unsat, mean tanh(llr/16), 1, 0, 0)
+#pragma unroll
+    for (int k = 0; k < FP_KC; ++k) {
+      const int c = tid + k * PROPOSE_THREADS;
+      if (c < C) {
+        const uint4 u = reinterpret_cast<const uint4*>(s_ci)[c];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        int d = 0;
+        uint32_t types = 0u;
+#pragma unroll
+        for (int e = 0; e < FP_DC; ++e) {
+          const int v = (int)(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
+          const int tu = s_tu[v];
+          s0 += s_th[v];
+          s1 += (float)((tu >> 1) & 1);
+          s2 += s_lut[tu >> 3];
+          d += v < V;
+          types |= (uint32_t)(tu & 7) << (3 * e);
+        }
+        s_ct[c] = types;
+        const float deg = (float)max(d, 1);
+        uint4 q;
+        q.x = pack_bf16((float)s_syn[c], s0 / deg);
+        q.y = pack_bf16(s1 / deg, s2 / deg);
+        q.z = pack_bf16(__ldg(pa.chk_lmean + c), 1.f);
+        q.w = 0u;
+        *reinterpret_cast<uint4*>(s_x + c * 8) = q;
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int layer = 1; layer <= 2; ++layer) {
+      bf16* s_m = layer == 1 ? s_a1 : s_a2;
+      // tile pass: this layer's messages
+      for (int tile = warp; tile < ntiles; tile += nwarps) {
+        float acc[8][4];
+        uint32_t ga[4][4];
+        const int r0 = tile * 16 + gq;
+        tile_embed(fr, s_x, r0, lane, tq, C, acc);
+        if (layer == 2) tile_update_halves(fr, FR_U1, s_bias, s_a1, r0, lane, tq, C, acc);
+        relu_to_a(acc, ga);
+        tile_message_halves(fr, layer == 1 ? FR_W1 : FR_W2, ga, r0, lane, tq, C, s_m);
+      }
+      __syncthreads();
+      // n_v = round(sum_{c in M(v)} m_c), a thread per variable and half of the channels
+      for (int i = tid; i < 2 * V; i += PROPOSE_THREADS) {
+        const int h = i >= V ? 1 : 0, v = i - h * V;
+        const uint2 u = reinterpret_cast<const uint2*>(s_vi)[v];
+        const int c[4] = {(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y & 0xffffu), (int)(u.y >> 16)};
+        const uint4* m = reinterpret_cast<const uint4*>(s_m + h * (C + 1) * 8);
+        uint4 r[DV];
+#pragma unroll
+        for (int j = 0; j < DV; ++j) r[j] = m[c[j]];
+        float n[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int j = 0; j < DV; ++j) {
+          float f[8];
+          unpack8(r[j], f);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) n[q] += f[q];
+        }
+        reinterpret_cast<uint4*>(s_n + h * (V + 1) * 8)[v] = pack8(n);
+      }
+      if (tid < 2) reinterpret_cast<uint4*>(s_n + tid * (V + 1) * 8)[V] = make_uint4(0u, 0u, 0u, 0u);
+      __syncthreads();
+      // a_c = sum_{v in N(c)} G[t_v] (n_v - m_c), a thread per check and half of the channels
+      for (int i = tid; i < 2 * C; i += PROPOSE_THREADS) {
+        const int h = i >= C ? 1 : 0, c = i - h * C;
+        const uint4 u = reinterpret_cast<const uint4*>(s_ci)[c];
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        const uint4* nh = reinterpret_cast<const uint4*>(s_n + h * (V + 1) * 8);
+        const unsigned char* gate = reinterpret_cast<const unsigned char*>(s_gate + (layer - 1) * 5 * ND + h * 8);
+        const uint32_t types = s_ct[c];
+        uint4* own = reinterpret_cast<uint4*>(s_m + h * (C + 1) * 8) + c;
+        float mc[8], a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        unpack8(*own, mc);
+#pragma unroll
+        for (int e = 0; e < FP_DC; ++e) {
+          const int v = (int)(e & 1 ? w[e >> 1] >> 16 : w[e >> 1] & 0xffffu);
+          float n[8], gt[8];
+          unpack8(nh[v], n);
+          const uint32_t off = (3 * e >= 5 ? types >> (3 * e - 5) : types << (5 - 3 * e)) & 0xe0u;  // type * 32 bytes
+          unpack8(*reinterpret_cast<const uint4*>(gate + off), gt);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) a[j] = fmaf(gt[j], n[j] - mc[j], a[j]);
+        }
+        *own = pack8(a);
+      }
+      __syncthreads();
+    }
+    // layer-2 update and the check readout o_c = O . g2^
+    for (int tile = warp; tile < ntiles; tile += nwarps) {
+      float acc[8][4];
+      uint32_t ga[4][4];
+      const int r0 = tile * 16 + gq;
+      tile_embed(fr, s_x, r0, lane, tq, C, acc);
+      tile_update_halves(fr, FR_U1, s_bias, s_a1, r0, lane, tq, C, acc);
+      tile_update_halves(fr, FR_U2, s_bias + NH, s_a2, r0, lane, tq, C, acc);
+      relu_to_a(acc, ga);
+      float oc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) mma_bf16(oc, ga[kk], fr[FR_O + kk * 64 + lane], fr[FR_O + kk * 64 + 32 + lane]);
+      if (tq == 0) {
+        if (r0 < C) s_o[r0] = oc[0];
+        if (r0 + 8 < C) s_o[r0 + 8] = oc[2];
+      }
+    }
+    if (tid == 0) s_o[C] = 0.f;
+    __syncthreads();
+    // variable readout
+#pragma unroll
+    for (int k = 0; k < FP_KV; ++k) {
+      const int v = tid + k * PROPOSE_THREADS;
+      if (v < V) {
+        const uint2 u = reinterpret_cast<const uint2*>(s_vi)[v];
+        const int c[4] = {(int)(u.x & 0xffffu), (int)(u.x >> 16), (int)(u.y & 0xffffu), (int)(u.y >> 16)};
+        float s = 0.f;
+        int d = 0;
+#pragma unroll
+        for (int j = 0; j < DV; ++j) {
+          s += s_o[c[j]];
+          d += c[j] < C;
+        }
+        const float deg = (float)max(d, 1);
+        const int tu = s_tu[v];
+        const float r = s / deg + (oz0 * th[k] + oz1 * (float)((tu >> 1) & 1) + oz2 * s_lut[tu >> 3] +
+                                   oz3 * __ldg(g.llr_feat + v)) + ob;
+        if (pa.logits) pa.logits[b * V + v] = r;
+        if (pa.gammas) pa.gammas[b * V + v] = pa.lo + (pa.hi - pa.lo) / (1.f + expf(-r));
+      }
+    }
+    b = next;
+    __syncthreads();
+  }
+}
+
 int grid_for(long long n, int threads = 256) {
   const long long b = (n + threads - 1) / threads;
   return (int)std::max(1LL, std::min(b, 148LL * 16));
@@ -798,6 +1119,10 @@ struct rbp_net {
   DevBuf<uint8_t> ty;
   int propose_smem = 0, propose_blocks = 0;
   ProposeArgs layout{};
+  DevBuf<uint16_t> chk_idx, var_idx;  // padded index rows of net_propose_fast_kernel
+  int fast_smem = 0;                  // 0: the graph does not fit that kernel
+  void (*fast_kernel)(NetGraph, ProposeArgs, FastArgs) = nullptr;
+  FastArgs fast{};
 
   NetGraph graph() const { return NetGraph{C, V, E, chk_ptr.p, chk_var.p, var_ptr.p, var_chk.p, llr_feat.p}; }
 
@@ -968,6 +1293,47 @@ int rbp_net_create(const rbp_graph* g, const float* llr, rbp_net** out) {
   int optin = 0, sms = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, n->device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device);
+  int max_dc = 0;
+  for (int c = 0; c < C; ++c) max_dc = std::max(max_dc, chk_ptr[c + 1] - chk_ptr[c]);
+  if (max_dc <= FP_DC && max_dv <= FP_DV && V <= FP_KV * PROPOSE_THREADS && C <= FP_KC * PROPOSE_THREADS) {
+    off = 0;
+    FastArgs& f = n->fast;
+    f.off_fr = take(FR_WORDS * 4);
+    f.off_gate = take(2 * 5 * ND * 2);
+    f.off_bias = take(2 * NH * 2);
+    f.off_lut = take(FP_LUT * 4);
+    f.off_ci = take(C * FP_DC * 2);
+    f.off_vi = take(V * FP_DV * 2);
+    f.off_x = take(C * 8 * 2);
+    f.off_a1 = take(2 * (C + 1) * 8 * 2);
+    f.off_a2 = take(2 * (C + 1) * 8 * 2);
+    f.off_n = take(std::max(2 * (V + 1) * 8 * 2, std::max(V, C) * 4 + 4));
+    f.off_tu = take(V + 1);
+    f.off_ct = take(C * 4);
+    f.off_syn = take(C + 1);
+    if (off <= optin) {
+      std::vector<uint16_t> ci((size_t)C * FP_DC, (uint16_t)V), vi((size_t)V * FP_DV, (uint16_t)C);
+      for (int c = 0; c < C; ++c)
+        for (int e = chk_ptr[c]; e < chk_ptr[c + 1]; ++e) ci[(size_t)c * FP_DC + e - chk_ptr[c]] = (uint16_t)edge_var[e];
+      for (int v = 0; v < V; ++v)
+        for (int k = g->var_ptr[v]; k < g->var_ptr[v + 1]; ++k)
+          vi[(size_t)v * FP_DV + k - g->var_ptr[v]] = (uint16_t)var_chk[k];
+      if ((rc = n->chk_idx.upload(ci.data(), ci.size())) || (rc = n->var_idx.upload(vi.data(), vi.size()))) {
+        delete n;
+        return rc;
+      }
+      n->fast_kernel = max_dv <= 3 ? net_propose_fast_kernel<3> : net_propose_fast_kernel<4>;
+      if (cudaFuncSetAttribute(reinterpret_cast<const void*>(n->fast_kernel),
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, off) != cudaSuccess) {
+        delete n;
+        return fail(RBP_ERR_CUDA, "rbp_net_create: cannot reserve shared memory for the inference kernel");
+      }
+      f.chk_idx = n->chk_idx.p;
+      f.var_idx = n->var_idx.p;
+      n->fast_smem = off;
+    }
+    off = n->propose_smem;
+  }
   if (small_graph && off <= optin) {
     if (cudaFuncSetAttribute(net_propose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, off) != cudaSuccess) {
       delete n;
@@ -1087,6 +1453,11 @@ int rbp_net_propose(rbp_net* n, int64_t B, const uint8_t* syn, const float* post
   pa.chk_lmean = n->chk_lmean.p;
   pa.graph16 = n->graph16.p;
   const int blocks = (int)std::min<long long>(B, n->propose_blocks);
+  if (n->fast_smem) {
+    n->fast_kernel<<<blocks, PROPOSE_THREADS, n->fast_smem, static_cast<cudaStream_t>(stream)>>>(n->graph(), pa, n->fast);
+    RBP_CUDA(cudaGetLastError());
+    return RBP_OK;
+  }
   net_propose_kernel<<<blocks, PROPOSE_THREADS, n->propose_smem, static_cast<cudaStream_t>(stream)>>>(n->graph(), pa);
   RBP_CUDA(cudaGetLastError());
   return RBP_OK;
