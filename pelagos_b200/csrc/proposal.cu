@@ -43,6 +43,7 @@
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -90,6 +91,30 @@ struct NetGraph {
 __device__ __forceinline__ float rbf(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float ldw(const bf16* p, int i) { return __bfloat162float(p[i]); }
 
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&p);
+}
+
+__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
+  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(p[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  uint4 q;
+  q.x = pack_bf16(f[0], f[1]);
+  q.y = pack_bf16(f[2], f[3]);
+  q.z = pack_bf16(f[4], f[5]);
+  q.w = pack_bf16(f[6], f[7]);
+  return q;
+}
+
 // Sum over the block (valid in thread 0); every thread of the block must call it.
 __device__ __forceinline__ float block_sum(float v, float* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -127,248 +152,528 @@ __global__ void feat_var_kernel(NetGraph g, long long B, const uint8_t* syn, con
   }
 }
 
-__global__ void feat_chk_kernel(NetGraph g, long long B, const uint8_t* syn, const float* z, const float* lmean,
-                                float* xr) {
-  const long long n = B * g.C;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long b = i / g.C;
-    const int c = (int)(i - b * g.C);
+// ------------------------------------------------------------------ rows (training path)
+//
+// A "row" is a check of a shot (row = b C + c), a "node" a variable of a shot.  A thread
+// owns a row: its 16- and 64-wide vectors stay in registers or pass through them one
+// channel at a time, weights come from shared memory as broadcasts (four per load), and
+// every sum runs in the order of a plain loop, in fp32.  What is kept for the backward
+// pass is what it needs: the rounded layer inputs (bf16 values, stored as such) and one
+// bit per channel for the relu; the 64-wide fp32 node states are recomputed, not stored.
+// Arrays are stored in 16-byte columns ([chunk][row]), so a warp's accesses are
+// contiguous.  With one thread per output element, each layer re-reading and re-writing
+// the node states (245 MB each for 1,024 shots of the 936 x 2,592 graph), a step of
+// 1,024 shots took 9.71 ms; now 2.08.
+
+// Gradients are summed in three steps: fp32 within a block (over its rows), one partial sum
+// per block in memory, and the blocks' sums in double.  With an atomic add per block the
+// additions to the running fp32 sum were the larger part of the error.
+constexpr int GRAD_BLOCKS = 148 * 4;               // at most so many blocks add to a parameter
+constexpr int GRAD_STRIDE = (N_PARAMS + 1 + 3) / 4 * 4;  // the loss comes after the parameters
+constexpr int RT = 128;       // threads (rows) of a row kernel's tile
+constexpr int SY = NH + 4;    // padded shared-memory rows of the gradient tiles
+constexpr int SX = ND + 4;
+
+struct NetWork {
+  float* z;                      // [nv][4] variable features
+  uint8_t* ty;                   // [nv] edge type
+  uint4* x;                      // [nc] check inputs x^ (8 bf16, 6 used)
+  uint4 *m1, *m2, *a1, *a2;      // [2][nc] messages, rounded aggregates
+  uint4 *n1, *n2;                // [2][nv] variable sums
+  uint4 *g1, *g2;                // [8][nc] round(relu(q)) of layers 1 and 2
+  unsigned long long *k1, *k2;   // [nc] bit j: q_j > 0
+  float *o, *dout;               // [nc]
+  float4 *da, *dm1, *dm2;        // [4][nc]
+  float4* dn;                    // [4][nv]
+};
+
+__device__ __forceinline__ void load16(const uint4* p, size_t n, size_t i, float (&f)[16]) {
+  float h[8];
+  unpack8(__ldg(p + i), h);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = h[j];
+  unpack8(__ldg(p + n + i), h);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[8 + j] = h[j];
+}
+
+__device__ __forceinline__ void load16(const float4* p, size_t n, size_t i, float (&f)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 v = __ldg(p + q * n + i);
+    f[4 * q] = v.x;
+    f[4 * q + 1] = v.y;
+    f[4 * q + 2] = v.z;
+    f[4 * q + 3] = v.w;
+  }
+}
+
+__device__ __forceinline__ void store16(uint4* p, size_t n, size_t i, const float (&f)[16]) {
+  float h[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = f[j];
+  p[i] = pack8(h);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) h[j] = f[8 + j];
+  p[n + i] = pack8(h);
+}
+
+__device__ __forceinline__ void store16(float4* p, size_t n, size_t i, const float (&f)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) p[q * n + i] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
+}
+
+// acc + sum_k f[k] w[k], k ascending, w 16 floats in shared memory
+__device__ __forceinline__ float dot16(const float (&f)[16], const float* w, float acc) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 v = *reinterpret_cast<const float4*>(w + 4 * q);
+    acc = fmaf(f[4 * q], v.x, acc);
+    acc = fmaf(f[4 * q + 1], v.y, acc);
+    acc = fmaf(f[4 * q + 2], v.z, acc);
+    acc = fmaf(f[4 * q + 3], v.w, acc);
+  }
+  return acc;
+}
+
+// acc[k] += y w[k]
+__device__ __forceinline__ void axpy16(float y, const float* w, float (&acc)[16]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 v = *reinterpret_cast<const float4*>(w + 4 * q);
+    acc[4 * q] = fmaf(y, v.x, acc[4 * q]);
+    acc[4 * q + 1] = fmaf(y, v.y, acc[4 * q + 1]);
+    acc[4 * q + 2] = fmaf(y, v.z, acc[4 * q + 2]);
+    acc[4 * q + 3] = fmaf(y, v.w, acc[4 * q + 3]);
+  }
+}
+
+// q0_j = E_j . x^
+__device__ __forceinline__ float embed(const float (&x)[8], const float* e) {
+  const float4 u = *reinterpret_cast<const float4*>(e);
+  const float2 v = *reinterpret_cast<const float2*>(e + 4);
+  float acc = fmaf(x[0], u.x, 0.f);
+  acc = fmaf(x[1], u.y, acc);
+  acc = fmaf(x[2], u.z, acc);
+  acc = fmaf(x[3], u.w, acc);
+  acc = fmaf(x[4], v.x, acc);
+  return fmaf(x[5], v.y, acc);
+}
+
+// Weights as fp32 in shared memory: E as [64][8], W (given [16][64]) transposed to [64][16].
+__device__ __forceinline__ void stage_e(const bf16* theta, float* s) {
+  for (int i = threadIdx.x; i < NH * 8; i += blockDim.x) s[i] = i % 8 < NX ? ldw(theta, P_E + i / 8 * NX + i % 8) : 0.f;
+}
+__device__ __forceinline__ void stage_t(const bf16* w, float* s) {
+  for (int i = threadIdx.x; i < NH * ND; i += blockDim.x) s[i] = ldw(w, i % ND * NH + i / ND);
+}
+__device__ __forceinline__ void stage(const bf16* w, int n, float* s) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s[i] = ldw(w, i);
+}
+
+// Forward of a row up to its next message (STAGE 1: x^ -> m1; 2: a1 -> m2) or readout (3: a2 -> o).
+template <int STAGE>
+__global__ void __launch_bounds__(RT) rows_forward_kernel(NetGraph g, unsigned nc, unsigned nv, NetWork w,
+                                                          const bf16* theta, const uint8_t* syn, const float* lmean) {
+  __shared__ __align__(16) float sE[NH * 8], sW[NH * ND], sU1[NH * ND], sU2[STAGE == 3 ? NH * ND : 4];
+  __shared__ float sb1[NH], sb2[NH], sO[NH];
+  __shared__ __align__(16) float sG[NTY * SX];
+  stage_e(theta, sE);
+  if (STAGE == 1) stage_t(theta + P_W1, sW);
+  if (STAGE == 2) stage_t(theta + P_W2, sW);
+  if (STAGE >= 2) {
+    stage(theta + P_U1, NH * ND, sU1);
+    stage(theta + P_B1, NH, sb1);
+    const bf16* G = theta + (STAGE == 2 ? P_G1 : P_G2);
+    for (int i = threadIdx.x; i < NTY * ND; i += RT) sG[i / ND * SX + i % ND] = ldw(G, i);
+  }
+  if (STAGE == 3) {
+    stage(theta + P_U2, NH * ND, sU2);
+    stage(theta + P_B2, NH, sb2);
+    stage(theta + P_O, NH, sO);
+  }
+  __syncthreads();
+  for (unsigned row = blockIdx.x * RT + threadIdx.x; row < nc; row += gridDim.x * RT) {
+    const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
     const int e0 = g.chk_ptr[c], e1 = g.chk_ptr[c + 1];
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-    for (int e = e0; e < e1; ++e) {
-      const float4 f = reinterpret_cast<const float4*>(z)[b * g.V + g.chk_var[e]];
-      s0 += f.x;
-      s1 += f.y;
-      s2 += f.z;
+    const size_t v0 = (size_t)b * g.V;
+    float x[8];
+    if constexpr (STAGE == 1) {
+      float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+      for (int e = e0; e < e1; ++e) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(w.z) + v0 + g.chk_var[e]);
+        s0 += f.x;
+        s1 += f.y;
+        s2 += f.z;
+      }
+      const float deg = (float)max(e1 - e0, 1);
+      x[0] = (float)(syn[row] & 1);
+      x[1] = s0 / deg;
+      x[2] = s1 / deg;
+      x[3] = s2 / deg;
+      x[4] = lmean[c];
+      x[5] = 1.f;
+      x[6] = x[7] = 0.f;
+      const uint4 q = pack8(x);
+      w.x[row] = q;
+      unpack8(q, x);
+    } else {
+      unpack8(__ldg(w.x + row), x);
     }
-    const float deg = (float)max(e1 - e0, 1);
-    float* o = xr + i * NX;
-    o[0] = (float)(syn[i] & 1);
-    o[1] = rbf(s0 / deg);
-    o[2] = rbf(s1 / deg);
-    o[3] = rbf(s2 / deg);
-    o[4] = rbf(lmean[c]);
-    o[5] = 1.f;
-  }
-}
-
-// ------------------------------------------------------------------ dense layers (training path)
-
-// Q[r, j] = sum_k round(act(X[r, k])) W[j, k] (+ bias[j]) (+ relu(R[r, j])), optionally rounded.
-template <int K, int N, bool XRELU, bool BIAS, bool RES, bool ROUND_OUT>
-__global__ void dense_fwd_kernel(long long n, const float* X, const bf16* W, const bf16* bias, const float* R,
-                                 float* Q) {
-  __shared__ float w[N * K];
-  __shared__ float bs[N];
-  for (int i = threadIdx.x; i < N * K; i += blockDim.x) w[i] = ldw(W, i);
-  if (BIAS)
-    for (int i = threadIdx.x; i < N; i += blockDim.x) bs[i] = ldw(bias, i);
-  __syncthreads();
-  const long long tot = n * N;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / N;
-    const int j = (int)(i - r * N);
-    const float* x = X + r * K;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < K; ++k) {
-      float xv = x[k];
-      if (XRELU) xv = fmaxf(xv, 0.f);
-      acc = fmaf(rbf(xv), w[j * K + k], acc);
-    }
-    if (BIAS) acc += bs[j];
-    if (RES) acc += fmaxf(R[i], 0.f);
-    Q[i] = ROUND_OUT ? rbf(acc) : acc;
-  }
-}
-
-// dX[r, k] (=|+=) sum_j dY[r, j] W[j, k]
-template <int K, int N, bool ACCUM>
-__global__ void dense_bwd_x_kernel(long long n, const float* dY, const bf16* W, float* dX) {
-  __shared__ float w[N * K];
-  for (int i = threadIdx.x; i < N * K; i += blockDim.x) w[i] = ldw(W, i);
-  __syncthreads();
-  const long long tot = n * K;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / K;
-    const int k = (int)(i - r * K);
-    const float* dy = dY + r * N;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int j = 0; j < N; ++j) acc = fmaf(dy[j], w[j * K + k], acc);
-    dX[i] = ACCUM ? dX[i] + acc : acc;
-  }
-}
-
-// dW[j, k] += sum_r dY[r, j] round(act(X[r, k])),  db[j] += sum_r dY[r, j].  256 threads per block.
-template <int K, int N, bool XRELU, bool BIAS>
-__global__ void __launch_bounds__(256) dense_bwd_w_kernel(long long n, const float* dY, const float* X, float* dW,
-                                                           float* db) {
-  constexpr int TR = 32;
-  constexpr int NP = N * K + (BIAS ? N : 0);
-  constexpr int PPT = (NP + 255) / 256;
-  __shared__ float sy[TR][N];
-  __shared__ float sx[TR][K];
-  float acc[PPT];
+    float a[16];
+    float al[16];  // layer 1's aggregates in stage 3
+    if constexpr (STAGE >= 2) {
+      // a_c = sum_{v in N(c)} G[t_v] (n_v - m_c)
+      const uint4* n = STAGE == 2 ? w.n1 : w.n2;
+      float mc[16];
+      load16(STAGE == 2 ? w.m1 : w.m2, nc, row, mc);
 #pragma unroll
-  for (int q = 0; q < PPT; ++q) acc[q] = 0.f;
-  const long long per = (n + gridDim.x - 1) / gridDim.x;
-  const long long r0 = blockIdx.x * per;
-  const long long r1 = min(n, r0 + per);
-  for (long long rb = r0; rb < r1; rb += TR) {
-    const int rows = (int)min((long long)TR, r1 - rb);
-    __syncthreads();
-    for (int i = threadIdx.x; i < TR * N; i += blockDim.x) {
-      const int rr = i / N, j = i - rr * N;
-      sy[rr][j] = rr < rows ? dY[(rb + rr) * N + j] : 0.f;
-    }
-    for (int i = threadIdx.x; i < TR * K; i += blockDim.x) {
-      const int rr = i / K, k = i - rr * K;
-      float xv = rr < rows ? X[(rb + rr) * K + k] : 0.f;
-      if (XRELU) xv = fmaxf(xv, 0.f);
-      sx[rr][k] = rbf(xv);
-    }
-    __syncthreads();
+      for (int k = 0; k < 16; ++k) a[k] = 0.f;
+      for (int e = e0; e < e1; ++e) {
+        const size_t v = v0 + g.chk_var[e];
+        float nf[16];
+        load16(n, nv, v, nf);
+        const float* gt = sG + __ldg(w.ty + v) * SX;
 #pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-      const int p = threadIdx.x + q * 256;
-      if (p < N * K) {
-        const int j = p / K, k = p - j * K;
-        float a = acc[q];
-        for (int rr = 0; rr < TR; ++rr) a = fmaf(sy[rr][j], sx[rr][k], a);
-        acc[q] = a;
-      } else if (BIAS && p < NP) {
-        const int j = p - N * K;
-        float a = acc[q];
-        for (int rr = 0; rr < TR; ++rr) a += sy[rr][j];
-        acc[q] = a;
+        for (int q = 0; q < 4; ++q) {
+          const float4 t = *reinterpret_cast<const float4*>(gt + 4 * q);
+          a[4 * q] = fmaf(t.x, nf[4 * q] - mc[4 * q], a[4 * q]);
+          a[4 * q + 1] = fmaf(t.y, nf[4 * q + 1] - mc[4 * q + 1], a[4 * q + 1]);
+          a[4 * q + 2] = fmaf(t.z, nf[4 * q + 2] - mc[4 * q + 2], a[4 * q + 2]);
+          a[4 * q + 3] = fmaf(t.w, nf[4 * q + 3] - mc[4 * q + 3], a[4 * q + 3]);
+        }
+      }
+      store16(STAGE == 2 ? w.a1 : w.a2, nc, row, a);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a[k] = rbf(a[k]);  // the layer's input
+      if constexpr (STAGE == 3) load16(w.a1, nc, row, al);
+    }
+    float m[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) m[k] = 0.f;
+    float o = 0.f;
+    unsigned long long mask = 0ull;
+#pragma unroll 1
+    for (int ch = 0; ch < NH / 8; ++ch) {
+      float gv[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int j = ch * 8 + i;
+        float q = embed(x, sE + j * 8);
+        if constexpr (STAGE == 2) q = dot16(a, sU1 + j * ND, 0.f) + sb1[j] + fmaxf(q, 0.f);
+        if constexpr (STAGE == 3) {
+          q = dot16(al, sU1 + j * ND, 0.f) + sb1[j] + fmaxf(q, 0.f);
+          q = dot16(a, sU2 + j * ND, 0.f) + sb2[j] + fmaxf(q, 0.f);
+        }
+        if (q > 0.f) mask |= 1ull << j;
+        gv[i] = rbf(fmaxf(q, 0.f));
+        if constexpr (STAGE < 3) axpy16(gv[i], sW + j * ND, m);
+        else o = fmaf(gv[i], sO[j], o);
+      }
+      if constexpr (STAGE == 2) w.g1[(size_t)ch * nc + row] = pack8(gv);
+      if constexpr (STAGE == 3) w.g2[(size_t)ch * nc + row] = pack8(gv);
+    }
+    if constexpr (STAGE == 1) store16(w.m1, nc, row, m);
+    if constexpr (STAGE == 2) {
+      store16(w.m2, nc, row, m);
+      w.k1[row] = mask;
+    }
+    if constexpr (STAGE == 3) {
+      w.o[row] = o;
+      w.k2[row] = mask;
+    }
+  }
+}
+
+// n_v = round(sum_{c in M(v)} m_c): a thread per node and half of the channels.
+__global__ void varsum_kernel(NetGraph g, unsigned nc, unsigned nv, const uint4* m, uint4* n) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nv) return;
+  const unsigned b = i / (unsigned)g.V, v = i - b * (unsigned)g.V;
+  const uint4* mh = m + (size_t)blockIdx.y * nc + (size_t)b * g.C;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int k = g.var_ptr[v]; k < g.var_ptr[v + 1]; ++k) {
+    float f[8];
+    unpack8(__ldg(mh + g.var_chk[k]), f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] += f[j];
+  }
+  n[(size_t)blockIdx.y * nv + i] = pack8(s);
+}
+
+// dn_v = G[t_v] sum_{c in M(v)} da_c: a thread per node and quarter of the channels.
+__global__ void dn_kernel(NetGraph g, unsigned nc, unsigned nv, const bf16* G, const uint8_t* ty, const float4* da,
+                          float4* dn) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nv) return;
+  const int q = blockIdx.y;
+  const unsigned b = i / (unsigned)g.V, v = i - b * (unsigned)g.V;
+  const float4* dc = da + (size_t)q * nc + (size_t)b * g.C;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k = g.var_ptr[v]; k < g.var_ptr[v + 1]; ++k) {
+    const float4 d = __ldg(dc + g.var_chk[k]);
+    s.x += d.x;
+    s.y += d.y;
+    s.z += d.z;
+    s.w += d.w;
+  }
+  const bf16* gt = G + ty[i] * ND + 4 * q;
+  dn[(size_t)q * nv + i] = make_float4(ldw(gt, 0) * s.x, ldw(gt, 1) * s.y, ldw(gt, 2) * s.z, ldw(gt, 3) * s.w);
+}
+
+// Backward of the aggregation and of the variable sums: dm_c = -(sum_v G[t_v]) da_c + sum_v dn_v and
+// dG[t] += da_c (n_v - m_c), a thread per row and quarter of the channels; the gate gradients stay
+// in the thread's registers over all its rows.
+__global__ void __launch_bounds__(512) dm_kernel(NetGraph g, unsigned nc, unsigned nv, const bf16* G, const uint8_t* ty,
+                                                 const uint4* m, const uint4* n, const float4* da, const float4* dn,
+                                                 float4* dm, float* dG) {
+  __shared__ __align__(16) float gs[NTY * ND];
+  __shared__ float acc[16][NTY * ND];
+  for (int i = threadIdx.x; i < NTY * ND; i += blockDim.x) gs[i] = ldw(G, i);
+  __syncthreads();
+  const int q = threadIdx.x & 3;
+  float part[NTY][4] = {};
+  for (unsigned row = blockIdx.x * 128 + (threadIdx.x >> 2); row < nc; row += gridDim.x * 128) {
+    const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
+    const size_t v0 = (size_t)b * g.V;
+    auto quad = [&](const uint4* p, size_t i) {  // channels 4q .. 4q+3 of a bf16 half row
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(p + i) + (q & 1));
+      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+      return make_float4(lo.x, lo.y, hi.x, hi.y);
+    };
+    const float4 mc = quad(m + (size_t)(q >> 1) * nc, row);
+    const float4 d = __ldg(da + (size_t)q * nc + row);
+    float4 gsum = make_float4(0.f, 0.f, 0.f, 0.f), s = gsum;
+    for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
+      const size_t v = v0 + g.chk_var[e];
+      const int t = __ldg(ty + v);
+      const float4 nf = quad(n + (size_t)(q >> 1) * nv, v);
+      const float4 gt = *reinterpret_cast<const float4*>(gs + t * ND + 4 * q);
+      const float4 dv = __ldg(dn + (size_t)q * nv + v);
+      gsum.x += gt.x;
+      gsum.y += gt.y;
+      gsum.z += gt.z;
+      gsum.w += gt.w;
+      s.x += dv.x;
+      s.y += dv.y;
+      s.z += dv.z;
+      s.w += dv.w;
+#pragma unroll
+      for (int tt = 0; tt < NTY; ++tt)
+        if (t == tt) {
+          part[tt][0] = fmaf(d.x, nf.x - mc.x, part[tt][0]);
+          part[tt][1] = fmaf(d.y, nf.y - mc.y, part[tt][1]);
+          part[tt][2] = fmaf(d.z, nf.z - mc.z, part[tt][2]);
+          part[tt][3] = fmaf(d.w, nf.w - mc.w, part[tt][3]);
+        }
+    }
+    dm[(size_t)q * nc + row] =
+        make_float4(-gsum.x * d.x + s.x, -gsum.y * d.y + s.y, -gsum.z * d.z + s.z, -gsum.w * d.w + s.w);
+  }
+#pragma unroll
+  for (int tt = 0; tt < NTY; ++tt)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float p = part[tt][i];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+      if ((threadIdx.x & 31) < 4) acc[threadIdx.x >> 5][tt * ND + 4 * q + i] = p;
+    }
+  __syncthreads();
+  if (threadIdx.x < NTY * ND) {
+    float s = 0.f;
+    for (int k = 0; k < 16; ++k) s += acc[k][threadIdx.x];
+    dG[(size_t)blockIdx.x * GRAD_STRIDE + threadIdx.x] = s;
+  }
+}
+
+// acc[i][k] += sum over the tile's rows of y[2 jp + i] x[4 kq + k]: a thread's 2 x 4 block of the
+// outer products summed over RT rows, 8 fmas per two shared-memory loads.
+__device__ __forceinline__ void outer_sum(const float* sy, const float* sx, int jp, int kq, float (&acc)[2][4]) {
+#pragma unroll 8
+  for (int r = 0; r < RT; ++r) {
+    const float2 y = *reinterpret_cast<const float2*>(sy + r * SY + 2 * jp);
+    const float4 x = *reinterpret_cast<const float4*>(sx + r * SX + 4 * kq);
+    acc[0][0] = fmaf(y.x, x.x, acc[0][0]);
+    acc[0][1] = fmaf(y.x, x.y, acc[0][1]);
+    acc[0][2] = fmaf(y.x, x.z, acc[0][2]);
+    acc[0][3] = fmaf(y.x, x.w, acc[0][3]);
+    acc[1][0] = fmaf(y.y, x.x, acc[1][0]);
+    acc[1][1] = fmaf(y.y, x.y, acc[1][1]);
+    acc[1][2] = fmaf(y.y, x.z, acc[1][2]);
+    acc[1][3] = fmaf(y.y, x.w, acc[1][3]);
+  }
+}
+
+// Backward of a row from the readout (STAGE 2) or from dm2 (1) to the aggregates' gradients da,
+// or from dm1 to the inputs (0), and the weight gradients of that stretch: per tile of RT rows
+// each 64-wide vector (dq, then the layer's input g) is laid in shared memory next to the
+// 16-wide one it multiplies, and a thread adds up its 2 x 4 block of the outer products.
+//   dq2_j = dout O_j [q2_j > 0],  dq1 = (dq2 + W2^T dm2) [q1 > 0],  dq0 = (dq1 + W1^T dm1) [q0 > 0]
+//   2: dO += dout g2, dU2 += dq2 a2^T, db2 += dq2, da = U2^T dq2
+//   1: dW2 += dm2 g1^T, dU1 += dq1 a1^T, db1 += dq1, da = U1^T dq1
+//   0: dW1 += dm1 g0^T, dE += dq0 x^T
+template <int STAGE>
+__global__ void __launch_bounds__(RT) rows_backward_kernel(NetGraph g, unsigned nc, NetWork w, const bf16* theta,
+                                                           const float* dr, float* grad) {
+  extern __shared__ __align__(16) float sm[];
+  float* sy = sm;                  // [RT][SY]
+  float* sx = sy + RT * SY;        // [RT][SX]
+  float* sO = sx + RT * SX;        // [64]
+  float* sW2 = sO + NH;            // [64][16] transposed (stages 1, 0)
+  float* sU = sW2 + (STAGE == 2 ? 0 : NH * ND);  // [64][16]: U2 or U1 (stages 2, 1)
+  float* sW1 = sU;                 // [64][16] transposed (stage 0)
+  float* sE = sW1 + NH * ND;       // [64][8] (stage 0)
+  stage(theta + P_O, NH, sO);
+  if (STAGE == 2) stage(theta + P_U2, NH * ND, sU);
+  if (STAGE == 1) stage(theta + P_U1, NH * ND, sU);
+  if (STAGE <= 1) stage_t(theta + P_W2, sW2);
+  if (STAGE == 0) {
+    stage_t(theta + P_W1, sW1);
+    stage_e(theta, sE);
+  }
+  const int t = threadIdx.x, jp = t >> 2, kq = t & 3;
+  float acc_y[2][4] = {}, acc_g[2][4] = {}, acc_b[2] = {};
+  for (unsigned r0 = blockIdx.x * RT; r0 < nc; r0 += gridDim.x * RT) {
+    const unsigned row = r0 + t;
+    const bool in = row < nc;
+    float da[16], dm2[16], dm1[16], x[8];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) da[k] = dm2[k] = dm1[k] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = 0.f;
+    float dout = 0.f;
+    unsigned long long k2 = 0ull, k1 = 0ull;
+    float* myx = sx + t * SX;
+    __syncthreads();  // the last tile's sums are done (first tile: the weights are staged)
+    if (in) {
+      k2 = w.k2[row];
+      if constexpr (STAGE == 2) {
+        const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
+        for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
+          const int v = g.chk_var[e];
+          dout += __ldg(dr + (size_t)b * g.V + v) / (float)max(g.var_ptr[v + 1] - g.var_ptr[v], 1);
+        }
+        w.dout[row] = dout;
+      } else {
+        dout = w.dout[row];
+        k1 = w.k1[row];
+        load16(w.dm2, nc, row, dm2);
+      }
+      if constexpr (STAGE == 0) {
+        load16(w.dm1, nc, row, dm1);
+        unpack8(__ldg(w.x + row), x);
       }
     }
-  }
+    // the 16-wide factor of dq: a2, a1 or x^
+    if constexpr (STAGE == 0) {
 #pragma unroll
-  for (int q = 0; q < PPT; ++q) {
-    const int p = threadIdx.x + q * 256;
-    if (p < N * K) atomicAdd(dW + p, acc[q]);
-    else if (BIAS && p < NP) atomicAdd(db + (p - N * K), acc[q]);
-  }
-}
-
-__global__ void relu_mask_kernel(long long n, const float* Q, float* dY) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    if (!(Q[i] > 0.f)) dY[i] = 0.f;
-}
-
-// ------------------------------------------------------------------ message passing (training path)
-
-// n[b, v, d] = round(sum_{c in M(v)} m[b, c, d])
-__global__ void varsum_kernel(NetGraph g, long long B, const float* m, float* nv) {
-  const long long tot = B * g.V * ND;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const int d = (int)(i % ND);
-    const long long bv = i / ND;
-    const long long b = bv / g.V;
-    const int v = (int)(bv - b * g.V);
-    float s = 0.f;
-    for (int k = g.var_ptr[v]; k < g.var_ptr[v + 1]; ++k) s += m[(b * g.C + g.var_chk[k]) * ND + d];
-    nv[i] = rbf(s);
-  }
-}
-
-// a[b, c, d] = sum_{v in N(c)} G[t_v, d] (n[b, v, d] - m[b, c, d])
-__global__ void agg_kernel(NetGraph g, long long B, const bf16* G, const uint8_t* ty, const float* m,
-                           const float* nv, float* a) {
-  __shared__ float gs[NTY * ND];
-  for (int i = threadIdx.x; i < NTY * ND; i += blockDim.x) gs[i] = ldw(G, i);
-  __syncthreads();
-  const long long tot = B * g.C * ND;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const int d = (int)(i % ND);
-    const long long bc = i / ND;
-    const long long b = bc / g.C;
-    const int c = (int)(bc - b * g.C);
-    const float mc = m[i];
-    float s = 0.f;
-    for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
-      const long long bv = b * g.V + g.chk_var[e];
-      s = fmaf(gs[ty[bv] * ND + d], nv[bv * ND + d] - mc, s);
-    }
-    a[i] = s;
-  }
-}
-
-// Backward of agg: dG += da (n_v - m_c) per edge type; dm = -(sum_v G[t_v]) da.
-__global__ void agg_bwd_kernel(NetGraph g, long long B, const bf16* G, const uint8_t* ty, const float* m,
-                               const float* nv, const float* da, float* dm, float* dG) {
-  __shared__ float gs[NTY * ND];
-  __shared__ float acc[NTY * ND];
-  for (int i = threadIdx.x; i < NTY * ND; i += blockDim.x) {
-    gs[i] = ldw(G, i);
-    acc[i] = 0.f;
-  }
-  __syncthreads();
-  const long long tot = B * g.C * ND;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const int d = (int)(i % ND);
-    const long long bc = i / ND;
-    const long long b = bc / g.C;
-    const int c = (int)(bc - b * g.C);
-    const float mc = m[i], dac = da[i];
-    float gsum = 0.f;
-    float part[NTY] = {0.f, 0.f, 0.f, 0.f};
-    for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
-      const long long bv = b * g.V + g.chk_var[e];
-      const int tt = ty[bv];
-      gsum += gs[tt * ND + d];
-      part[tt] = fmaf(dac, nv[bv * ND + d] - mc, part[tt]);
-    }
-    dm[i] = -gsum * dac;
+      for (int k = 0; k < 16; ++k) myx[k] = k < 8 ? x[k & 7] : 0.f;
+    } else {
+      float a[16] = {};
+      if (in) load16(STAGE == 2 ? w.a2 : w.a1, nc, row, a);
 #pragma unroll
-    for (int tt = 0; tt < NTY; ++tt)
-      if (part[tt] != 0.f) atomicAdd(&acc[tt * ND + d], part[tt]);
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4*>(myx + 4 * q) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+    }
+#pragma unroll 1
+    for (int j0 = 0; j0 < NH; j0 += 4) {
+      float dq[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int j = j0 + i;
+        float d = (k2 >> j) & 1ull ? dout * sO[j] : 0.f;
+        if constexpr (STAGE <= 1) d = (k1 >> j) & 1ull ? d + dot16(dm2, sW2 + j * ND, 0.f) : 0.f;
+        if constexpr (STAGE == 0) {
+          d += dot16(dm1, sW1 + j * ND, 0.f);
+          if (!(embed(x, sE + j * 8) > 0.f)) d = 0.f;
+        } else {
+          axpy16(d, sU + j * ND, da);
+        }
+        dq[i] = d;
+      }
+      *reinterpret_cast<float4*>(sy + t * SY + j0) = make_float4(dq[0], dq[1], dq[2], dq[3]);
+    }
+    if constexpr (STAGE >= 1) {
+      if (in) store16(w.da, nc, row, da);
+    }
+    __syncthreads();
+    if (STAGE > 0 || kq < 2) outer_sum(sy, sx, jp, kq, acc_y);
+    if constexpr (STAGE >= 1) {  // biases: a quarter of the rows per kq
+#pragma unroll 8
+      for (int r = kq; r < RT; r += 4) {
+        const float2 y = *reinterpret_cast<const float2*>(sy + r * SY + 2 * jp);
+        acc_b[0] += y.x;
+        acc_b[1] += y.y;
+      }
+    }
+    __syncthreads();
+    // the layer's input g and its factor: dout, dm2 or dm1
+#pragma unroll 1
+    for (int ch = 0; ch < NH / 8; ++ch) {
+      float gv[8] = {};
+      if constexpr (STAGE == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) gv[i] = in ? rbf(fmaxf(embed(x, sE + (ch * 8 + i) * 8), 0.f)) : 0.f;
+      } else if (in) {
+        unpack8(__ldg((STAGE == 2 ? w.g2 : w.g1) + (size_t)ch * nc + row), gv);
+      }
+      float* y = sy + t * SY + ch * 8;
+      *reinterpret_cast<float4*>(y) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+      *reinterpret_cast<float4*>(y + 4) = make_float4(gv[4], gv[5], gv[6], gv[7]);
+    }
+    if constexpr (STAGE == 2) {
+      myx[0] = dout;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) myx[k] = STAGE == 1 ? dm2[k] : dm1[k];
+    }
+    __syncthreads();
+    if constexpr (STAGE == 2) {
+#pragma unroll 8
+      for (int r = kq; r < RT; r += 4) {
+        const float2 y = *reinterpret_cast<const float2*>(sy + r * SY + 2 * jp);
+        const float d = sx[r * SX];
+        acc_g[0][0] = fmaf(d, y.x, acc_g[0][0]);
+        acc_g[1][0] = fmaf(d, y.y, acc_g[1][0]);
+      }
+    } else {
+      outer_sum(sy, sx, jp, kq, acc_g);
+    }
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < NTY * ND; i += blockDim.x)
-    if (acc[i] != 0.f) atomicAdd(dG + i, acc[i]);
+  float* out = grad + (size_t)blockIdx.x * GRAD_STRIDE;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int j = 2 * jp + i;
+    // biases and dO: the four kq threads of a channel pair hold a quarter of the rows each
+    float q = acc_b[i], o = acc_g[i][0];
+#pragma unroll
+    for (int m = 1; m < 4; m <<= 1) {
+      q += __shfl_xor_sync(0xffffffffu, q, m);
+      o += __shfl_xor_sync(0xffffffffu, o, m);
+    }
+    if (STAGE >= 1 && kq == 0) out[(STAGE == 2 ? P_B2 : P_B1) + j] = q;
+    if (STAGE == 2 && kq == 0) out[P_O + j] = o;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if constexpr (STAGE >= 1) out[(STAGE == 2 ? P_U2 : P_U1) + j * ND + 4 * kq + k] = acc_y[i][k];
+      else if (4 * kq + k < NX) out[P_E + j * NX + 4 * kq + k] = acc_y[i][k];
+      if constexpr (STAGE <= 1) out[(STAGE == 1 ? P_W2 : P_W1) + (4 * kq + k) * NH + j] = acc_g[i][k];
+    }
+  }
 }
-
-// dn[b, v, d] = G[t_v, d] sum_{c in M(v)} da[b, c, d]
-__global__ void dn_kernel(NetGraph g, long long B, const bf16* G, const uint8_t* ty, const float* da, float* dn) {
-  __shared__ float gs[NTY * ND];
-  for (int i = threadIdx.x; i < NTY * ND; i += blockDim.x) gs[i] = ldw(G, i);
-  __syncthreads();
-  const long long tot = B * g.V * ND;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const int d = (int)(i % ND);
-    const long long bv = i / ND;
-    const long long b = bv / g.V;
-    const int v = (int)(bv - b * g.V);
-    float s = 0.f;
-    for (int k = g.var_ptr[v]; k < g.var_ptr[v + 1]; ++k) s += da[(b * g.C + g.var_chk[k]) * ND + d];
-    dn[i] = gs[ty[bv] * ND + d] * s;
-  }
-}
-
-// dm[b, c, d] += sum_{v in N(c)} dn[b, v, d]
-__global__ void varsum_bwd_kernel(NetGraph g, long long B, const float* dn, float* dm) {
-  const long long tot = B * g.C * ND;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const int d = (int)(i % ND);
-    const long long bc = i / ND;
-    const long long b = bc / g.C;
-    const int c = (int)(bc - b * g.C);
-    float s = 0.f;
-    for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) s += dn[(b * g.V + g.chk_var[e]) * ND + d];
-    dm[i] += s;
-  }
+constexpr int rows_backward_smem(int stage) {
+  return (RT * SY + RT * SX + NH + (stage == 2 ? 1 : 2) * NH * ND + (stage == 0 ? NH * 8 : 0)) * 4;
 }
 
 // ------------------------------------------------------------------ readout and loss (training path)
 
 // r = sum_{c in M(v)} o_c / deg_v + Oz.z_v + ob.  With targets: the weighted
-// logistic loss (summed into *loss, divided by B V), dr, and the Oz / ob gradients.
+// logistic loss (divided by B V), dr, and the Oz / ob gradients, as the block's partial sums.
 __global__ void __launch_bounds__(256) readout_kernel(NetGraph g, long long B, const bf16* theta, const float* o,
                                                       const float* z, const uint8_t* y, float w_neg, float* r,
-                                                      float* dr, float* loss, float* grad) {
+                                                      float* dr, float* grad) {
   __shared__ float red[32];
   const float oz0 = ldw(theta, P_OZ), oz1 = ldw(theta, P_OZ + 1), oz2 = ldw(theta, P_OZ + 2),
               oz3 = ldw(theta, P_OZ + 3), ob = ldw(theta, P_OB);
@@ -400,25 +705,31 @@ __global__ void __launch_bounds__(256) readout_kernel(NetGraph g, long long B, c
   }
   if (!y) return;  // uniform over the block
   const float vals[6] = {l_acc * inv_n, g0, g1, g2, g3, gb};
-  float* dst[6] = {loss, grad + P_OZ, grad + P_OZ + 1, grad + P_OZ + 2, grad + P_OZ + 3, grad + P_OB};
+  float* out = grad + (size_t)blockIdx.x * GRAD_STRIDE;
+  const int dst[6] = {N_PARAMS, P_OZ, P_OZ + 1, P_OZ + 2, P_OZ + 3, P_OB};
   for (int q = 0; q < 6; ++q) {
     const float t = block_sum(vals[q], red);
-    if (threadIdx.x == 0) atomicAdd(dst[q], t);
+    if (threadIdx.x == 0) out[dst[q]] = t;
   }
 }
 
-// do[b, c] = sum_{v in N(c)} dr[b, v] / deg_v
-__global__ void readout_bwd_kernel(NetGraph g, long long B, const float* dr, float* dout) {
-  const long long tot = B * g.C;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
-    const long long b = i / g.C;
-    const int c = (int)(i - b * g.C);
-    float s = 0.f;
-    for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
-      const int v = g.chk_var[e];
-      s += dr[b * g.V + v] / (float)max(g.var_ptr[v + 1] - g.var_ptr[v], 1);
-    }
-    dout[i] = s;
+// The blocks' partial sums of each parameter (and of the loss), added in double: 8 warps share
+// 32 parameters.  rows / gates / vars: blocks of the kernels behind a parameter.
+__global__ void __launch_bounds__(256) grad_sum_kernel(const float* partial, int rows, int gates, int vars, float* grad,
+                                                       float* loss) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+  const bool gate = (p >= P_G1 && p < P_U1) || (p >= P_G2 && p < P_U2);
+  const int n = p > N_PARAMS ? 0 : (gate ? gates : (p >= P_OZ ? vars : rows));
+  double s = 0.0;
+#pragma unroll 4
+  for (int k = warp; k < n; k += 8) s += (double)partial[(size_t)k * GRAD_STRIDE + p];
+  part[warp][lane] = s;
+  __syncthreads();
+  if (warp == 0 && p <= N_PARAMS) {
+    for (int k = 1; k < 8; ++k) s += part[k][lane];
+    if (p < N_PARAMS) grad[p] = (float)s;
+    else *loss = (float)s;
   }
 }
 
@@ -468,31 +779,7 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&p);
-}
-
 __device__ __forceinline__ float sw_f(const bf16* w, int i) { return __bfloat162float(w[i]); }
-
-__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
-  const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __bfloat1622float2(p[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-  uint4 q;
-  q.x = pack_bf16(f[0], f[1]);
-  q.y = pack_bf16(f[2], f[3]);
-  q.z = pack_bf16(f[4], f[5]);
-  q.w = pack_bf16(f[6], f[7]);
-  return q;
-}
 
 // B operands of the tensor-core layers, stored per fragment so that a warp
 // reads each fragment as 32 consecutive words (lane l at word l): no bank
@@ -1115,8 +1402,10 @@ struct rbp_net {
   DevBuf<bf16> theta_bf;
   long long step = 0;
   long long ws_B = 0;
-  DevBuf<float> z, xr, q0, q1, q2, m1, m2, n1, n2, a1, a2, o, r, dr, dg, da, dn, dm, dout;
-  DevBuf<uint8_t> ty;
+  DevBuf<uint4> slab;           // the training workspace, one allocation
+  NetWork ws{};
+  float *r = nullptr, *dr = nullptr;
+  float* partial = nullptr;     // [GRAD_BLOCKS][GRAD_STRIDE]
   int propose_smem = 0, propose_blocks = 0;
   ProposeArgs layout{};
   DevBuf<uint16_t> chk_idx, var_idx;  // padded index rows of net_propose_fast_kernel
@@ -1129,77 +1418,72 @@ struct rbp_net {
   int workspace(long long B) {
     if (B <= ws_B) return RBP_OK;
     const size_t nc = (size_t)B * C, nv = (size_t)B * V;
-    int rc;
-    if ((rc = z.upload(nullptr, nv * NF)) || (rc = ty.upload(nullptr, nv)) || (rc = xr.upload(nullptr, nc * NX)) ||
-        (rc = q0.upload(nullptr, nc * NH)) || (rc = q1.upload(nullptr, nc * NH)) ||
-        (rc = q2.upload(nullptr, nc * NH)) || (rc = m1.upload(nullptr, nc * ND)) ||
-        (rc = m2.upload(nullptr, nc * ND)) || (rc = n1.upload(nullptr, nv * ND)) ||
-        (rc = n2.upload(nullptr, nv * ND)) || (rc = a1.upload(nullptr, nc * ND)) ||
-        (rc = a2.upload(nullptr, nc * ND)) || (rc = o.upload(nullptr, nc)) || (rc = r.upload(nullptr, nv)) ||
-        (rc = dr.upload(nullptr, nv)) || (rc = dg.upload(nullptr, nc * NH)) || (rc = da.upload(nullptr, nc * ND)) ||
-        (rc = dn.upload(nullptr, nv * ND)) || (rc = dm.upload(nullptr, nc * ND)) || (rc = dout.upload(nullptr, nc))) {
-      ws_B = 0;
-      return rc;
+    ws_B = 0;
+    unsigned char* base = nullptr;
+    size_t off = 0;
+    auto take = [&](auto*& p, size_t count) {
+      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + off);
+      off += (count * sizeof(*p) + 255) / 256 * 256;
+    };
+    for (int pass = 0; pass < 2; ++pass) {  // sizes, then places
+      if (pass == 1) {
+        const int rc = slab.upload(nullptr, off / sizeof(uint4));
+        if (rc != RBP_OK) return rc;
+        base = reinterpret_cast<unsigned char*>(slab.p);
+        off = 0;
+      }
+      take(ws.z, nv * NF);
+      take(ws.ty, nv);
+      take(ws.x, nc);
+      for (uint4** p : {&ws.m1, &ws.m2, &ws.a1, &ws.a2}) take(*p, nc * 2);
+      for (uint4** p : {&ws.n1, &ws.n2}) take(*p, nv * 2);
+      for (uint4** p : {&ws.g1, &ws.g2}) take(*p, nc * 8);
+      for (unsigned long long** p : {&ws.k1, &ws.k2}) take(*p, nc);
+      for (float** p : {&ws.o, &ws.dout}) take(*p, nc);
+      for (float4** p : {&ws.da, &ws.dm1, &ws.dm2}) take(*p, nc * 4);
+      take(ws.dn, nv * 4);
+      for (float** p : {&r, &dr}) take(*p, nv);
+      take(partial, (size_t)GRAD_BLOCKS * GRAD_STRIDE);
     }
     ws_B = B;
     return RBP_OK;
   }
 
-  // Training-path forward; leaves every activation in the workspace.
+  // Training-path forward; leaves what the backward pass needs in the workspace.
   void forward(long long B, const uint8_t* syn, const float* post, cudaStream_t st) {
     const NetGraph g = graph();
-    const long long nc = B * C, nv = B * V;
+    const NetWork& w = ws;
+    const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
+    // weights are staged once per block: the resident blocks loop over their rows
+    const unsigned rows = std::min<unsigned>((nc + RT - 1) / RT, 148 * 6);
+    const dim3 halves((nv + 255) / 256, 2);
     const bf16* t = theta_bf.p;
-    feat_var_kernel<<<grid_for(nv), 256, 0, st>>>(g, B, syn, post, z.p, ty.p);
-    feat_chk_kernel<<<grid_for(nc), 256, 0, st>>>(g, B, syn, z.p, chk_lmean.p, xr.p);
-    dense_fwd_kernel<NX, NH, false, false, false, false><<<grid_for(nc * NH), 256, 0, st>>>(nc, xr.p, t + P_E, nullptr,
-                                                                                             nullptr, q0.p);
-    // layer 1
-    dense_fwd_kernel<NH, ND, true, false, false, true><<<grid_for(nc * ND), 256, 0, st>>>(nc, q0.p, t + P_W1, nullptr,
-                                                                                           nullptr, m1.p);
-    varsum_kernel<<<grid_for(nv * ND), 256, 0, st>>>(g, B, m1.p, n1.p);
-    agg_kernel<<<grid_for(nc * ND), 256, 0, st>>>(g, B, t + P_G1, ty.p, m1.p, n1.p, a1.p);
-    dense_fwd_kernel<ND, NH, false, true, true, false><<<grid_for(nc * NH), 256, 0, st>>>(nc, a1.p, t + P_U1, t + P_B1,
-                                                                                           q0.p, q1.p);
-    // layer 2
-    dense_fwd_kernel<NH, ND, true, false, false, true><<<grid_for(nc * ND), 256, 0, st>>>(nc, q1.p, t + P_W2, nullptr,
-                                                                                           nullptr, m2.p);
-    varsum_kernel<<<grid_for(nv * ND), 256, 0, st>>>(g, B, m2.p, n2.p);
-    agg_kernel<<<grid_for(nc * ND), 256, 0, st>>>(g, B, t + P_G2, ty.p, m2.p, n2.p, a2.p);
-    dense_fwd_kernel<ND, NH, false, true, true, false><<<grid_for(nc * NH), 256, 0, st>>>(nc, a2.p, t + P_U2, t + P_B2,
-                                                                                           q1.p, q2.p);
-    // check readout
-    dense_fwd_kernel<NH, 1, true, false, false, false><<<grid_for(nc), 256, 0, st>>>(nc, q2.p, t + P_O, nullptr,
-                                                                                      nullptr, o.p);
+    feat_var_kernel<<<grid_for(nv), 256, 0, st>>>(g, B, syn, post, w.z, w.ty);
+    rows_forward_kernel<1><<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
+    varsum_kernel<<<halves, 256, 0, st>>>(g, nc, nv, w.m1, w.n1);
+    rows_forward_kernel<2><<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
+    varsum_kernel<<<halves, 256, 0, st>>>(g, nc, nv, w.m2, w.n2);
+    rows_forward_kernel<3><<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
   }
 
-  // Backward of one layer.  On entry dg = dL/d relu(q); on exit dg = dL/d relu(q_prev).
-  void layer_backward(long long B, const float* q_prev, const float* q, const float* a, const float* m,
-                      const float* n, int pw, int pg, int pu, int pb, cudaStream_t st) {
+  // Gradients of everything behind the readout (dr), summed with the readout's own into grad and loss.
+  void backward(long long B, int vars, cudaStream_t st) {
     const NetGraph g = graph();
-    const long long nc = B * C, nv = B * V;
+    const NetWork& w = ws;
+    const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
+    const dim3 quarters((nv + 255) / 256, 4);
+    const int tiles = (int)std::min<unsigned>((nc + RT - 1) / RT, GRAD_BLOCKS);  // four resident blocks per SM
+    const int gather = (int)std::min<unsigned>((nc + 127) / 128, GRAD_BLOCKS);
+    float* pg = partial;
     const bf16* t = theta_bf.p;
-    relu_mask_kernel<<<grid_for(nc * NH), 256, 0, st>>>(nc * NH, q, dg.p);  // dg = dL/dq
-    dense_bwd_w_kernel<ND, NH, false, true><<<148 * 2, 256, 0, st>>>(nc, dg.p, a, grad.p + pu, grad.p + pb);
-    dense_bwd_x_kernel<ND, NH, false><<<grid_for(nc * ND), 256, 0, st>>>(nc, dg.p, t + pu, da.p);
-    agg_bwd_kernel<<<grid_for(nc * ND), 256, 0, st>>>(g, B, t + pg, ty.p, m, n, da.p, dm.p, grad.p + pg);
-    dn_kernel<<<grid_for(nv * ND), 256, 0, st>>>(g, B, t + pg, ty.p, da.p, dn.p);
-    varsum_bwd_kernel<<<grid_for(nc * ND), 256, 0, st>>>(g, B, dn.p, dm.p);
-    dense_bwd_w_kernel<NH, ND, true, false><<<148 * 2, 256, 0, st>>>(nc, dm.p, q_prev, grad.p + pw, nullptr);
-    dense_bwd_x_kernel<NH, ND, true><<<grid_for(nc * NH), 256, 0, st>>>(nc, dm.p, t + pw, dg.p);  // + residual
-  }
-
-  void backward(long long B, cudaStream_t st) {
-    const NetGraph g = graph();
-    const long long nc = B * C;
-    const bf16* t = theta_bf.p;
-    readout_bwd_kernel<<<grid_for(nc), 256, 0, st>>>(g, B, dr.p, dout.p);
-    dense_bwd_w_kernel<NH, 1, true, false><<<148 * 2, 256, 0, st>>>(nc, dout.p, q2.p, grad.p + P_O, nullptr);
-    dense_bwd_x_kernel<NH, 1, false><<<grid_for(nc * NH), 256, 0, st>>>(nc, dout.p, t + P_O, dg.p);
-    layer_backward(B, q1.p, q2.p, a2.p, m2.p, n2.p, P_W2, P_G2, P_U2, P_B2, st);
-    layer_backward(B, q0.p, q1.p, a1.p, m1.p, n1.p, P_W1, P_G1, P_U1, P_B1, st);
-    relu_mask_kernel<<<grid_for(nc * NH), 256, 0, st>>>(nc * NH, q0.p, dg.p);
-    dense_bwd_w_kernel<NX, NH, false, false><<<148 * 2, 256, 0, st>>>(nc, dg.p, xr.p, grad.p + P_E, nullptr);
+    rows_backward_kernel<2><<<tiles, RT, rows_backward_smem(2), st>>>(g, nc, w, t, dr, pg);
+    dn_kernel<<<quarters, 256, 0, st>>>(g, nc, nv, t + P_G2, w.ty, w.da, w.dn);
+    dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G2, w.ty, w.m2, w.n2, w.da, w.dn, w.dm2, pg + P_G2);
+    rows_backward_kernel<1><<<tiles, RT, rows_backward_smem(1), st>>>(g, nc, w, t, dr, pg);
+    dn_kernel<<<quarters, 256, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.da, w.dn);
+    dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.m1, w.n1, w.da, w.dn, w.dm1, pg + P_G1);
+    rows_backward_kernel<0><<<tiles, RT, rows_backward_smem(0), st>>>(g, nc, w, t, dr, pg);
+    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 256, 0, st>>>(pg, tiles, gather, vars, grad.p, loss.p);
   }
 };
 
@@ -1256,6 +1540,13 @@ int rbp_net_create(const rbp_graph* g, const float* llr, rbp_net** out) {
     return rc;
   }
   to_bf16_kernel<<<4, 256>>>(N_PARAMS, n->theta.p, n->theta_bf.p);
+  for (const void* k : {reinterpret_cast<const void*>(rows_backward_kernel<0>),
+                        reinterpret_cast<const void*>(rows_backward_kernel<1>),
+                        reinterpret_cast<const void*>(rows_backward_kernel<2>)})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_backward_smem(0)) != cudaSuccess) {
+      delete n;
+      return fail(RBP_ERR_CUDA, "rbp_net_create: cannot reserve shared memory for the training kernels");
+    }
   // inference kernel shared memory (see net_propose_kernel)
   int off = 0;
   auto take = [&](int bytes) {
@@ -1389,8 +1680,8 @@ int rbp_net_forward(rbp_net* n, int64_t B, const uint8_t* syn, const float* post
   if ((rc = n->workspace(B))) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   n->forward(B, syn, post, st);
-  readout_kernel<<<grid_for(B * n->V), 256, 0, st>>>(n->graph(), B, n->theta_bf.p, n->o.p, n->z.p, nullptr, 0.f,
-                                                      logits, nullptr, nullptr, nullptr);
+  readout_kernel<<<grid_for(B * n->V), 256, 0, st>>>(n->graph(), B, n->theta_bf.p, n->ws.o, n->ws.z, nullptr, 0.f,
+                                                      logits, nullptr, nullptr);
   RBP_CUDA(cudaGetLastError());
   return RBP_OK;
 }
@@ -1405,12 +1696,11 @@ int rbp_net_train_step(rbp_net* n, int64_t B, const uint8_t* syn, const float* p
   int rc;
   if ((rc = n->workspace(B))) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  RBP_CUDA(cudaMemsetAsync(n->grad.p, 0, N_PARAMS * sizeof(float), st));
-  RBP_CUDA(cudaMemsetAsync(n->loss.p, 0, sizeof(float), st));
   n->forward(B, syn, post, st);
-  readout_kernel<<<grid_for(B * n->V), 256, 0, st>>>(n->graph(), B, n->theta_bf.p, n->o.p, n->z.p, target,
-                                                      hp->w_neg, n->r.p, n->dr.p, n->loss.p, n->grad.p);
-  n->backward(B, st);
+  const int vars = std::min(grid_for(B * n->V), GRAD_BLOCKS);
+  readout_kernel<<<vars, 256, 0, st>>>(n->graph(), B, n->theta_bf.p, n->ws.o, n->ws.z, target, hp->w_neg, n->r,
+                                       n->dr, n->partial);
+  n->backward(B, vars, st);
   if (loss) RBP_CUDA(cudaMemcpyAsync(loss, n->loss.p, sizeof(float), cudaMemcpyDeviceToDevice, st));
   if (grads) RBP_CUDA(cudaMemcpyAsync(grads, n->grad.p, N_PARAMS * sizeof(float), cudaMemcpyDeviceToDevice, st));
   if (hp->lr > 0.f) {
