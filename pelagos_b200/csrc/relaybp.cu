@@ -70,6 +70,9 @@ struct rbp_decoder {
   // launch shapes: shape[0] for launches that skip the relay legs (pre-iterations
   // only, so a shot's latency is bounded by pre_iter), shape[1] for the others
   Launch shape[2];
+  bool automatic[2] = {true, true};  // shape[k] is the library's choice: larger batches may run `bulk`
+  Launch bulk{};
+  int64_t bulk_from = INT64_MAX;     // batch size from which `bulk` runs
   int sm_count = 0;
   size_t max_smem = 0;
 };
@@ -315,6 +318,58 @@ int choose_launch(int C, int V, int slots, int vslots, int rows, int msg_type, i
   return RBP_OK;
 }
 
+// The library's own choice of shape: `small` for batches below `bulk_from`, `bulk` from there on.
+//
+// One group per block, compiled for two resident blocks per SM, with the fewest owned
+// variables per thread that its register budget allows: the steady iteration of one shot
+// is shortest then, and what a batch waits for is mostly its slowest shots.  Against as
+// many groups per block as fit at three variables per thread (the rule for everything
+// else), us: [[144,12,12]] code capacity 20,001 shots 160 threads 1,846 (mean of three
+// seeds) against 2,242; 216 variables 65,536 shots 4,714 against 7,198; 648 variables 30,000 shots
+// 5,417 against 7,393; 1,728 variables 30,000 shots 6,721 against 8,990; [[72,12,6]] 100 shots 206
+// against 303.  A few more threads where they save a round of check rows (432 rows of 1,080
+// variables: 448 threads 6,125, 384 threads 6,567).  Two exceptions:
+//  * beyond four variables per thread (V > 2,048) a lone shot is no faster than with the
+//    other rule's larger group (2,592 variables, 2,000 shots: 4,622 against 4,530), so that one
+//    keeps batches of up to 16 shots per resident group; 65,536 shots: 15,300 against 20,200;
+//  * groups of one warp (V <= 96) need no barrier and win once they are four times
+//    oversubscribed: [[72,12,6]], 65,536 shots 964 against 1,171, but 8,192 shots 523 against 419.
+// A code whose blocks do not fit twice on an SM keeps the other rule.
+int choose_automatic(int C, int V, int slots, int vslots, int rows, int msg_type, size_t max_smem, int sm_count,
+                     Launch* small, Launch* bulk, int64_t* bulk_from, const char* who) {
+  *bulk_from = INT64_MAX;
+  auto other_rule = [&]() {
+    return choose_launch(C, V, slots, vslots, rows, msg_type, default_group_threads(C, V), 0, max_smem, sm_count, small,
+                         who);
+  };
+  auto two_per_sm = [&](int G, Launch* out) {
+    return choose_launch(C, V, slots, vslots, rows, msg_type, G, 1, max_smem, sm_count, out, who, 1, 2) == RBP_OK &&
+           out->blocks >= 2 * sm_count;
+  };
+  for (int vpt : rbpk::kVptChoices) {
+    if (slots > 16) break;
+    int G = std::max(32, (V + vpt - 1) / vpt + 31) / 32 * 32;
+    const int most = rbpk::max_block_threads2(vpt);
+    if (G > most || vpt_for(V, G) != vpt) continue;
+    const int rounds = (C + G - 1) / G;
+    if (rounds > 1) {
+      const int wider = ((C + rounds - 2) / (rounds - 1) + 31) / 32 * 32;
+      if (wider <= most && wider * 4 <= G * 5 && vpt_for(V, wider) == vpt) G = wider;
+    }
+    Launch two{};
+    if (!two_per_sm(G, &two)) break;
+    if (vpt > 4) {
+      *bulk = two;
+      *bulk_from = 16LL * two.blocks;
+      break;
+    }
+    *small = two;
+    if (V <= 96 && two_per_sm(32, bulk)) *bulk_from = 4LL * bulk->blocks;
+    return RBP_OK;
+  }
+  return other_rule();
+}
+
 int check_batch(const char* who, int64_t B, const rbp_batch* in, const rbp_outputs* out, const rbp_params& p,
                 int n_alpha) {
   const std::string w(who);
@@ -548,9 +603,23 @@ int rbp_decoder_configure_kind(rbp_decoder* d, int32_t kind, int32_t group_threa
   const int nshots = shots_per_group > 0 ? shots_per_group : 1;
   // groups_per_block 0 (default) or -1: the multi-group kernel with as many one-shot groups
   // per block as fit; 1, or two shots per group: the block-per-group kernel
+  const bool automatic = group_threads <= 0 && groups_per_block == 0 && nshots == 1 && blocks_per_sm == 0;
   if (groups_per_block < 0) {
     if (nshots != 1) return fail(RBP_ERR_ARGUMENT, "rbp_decoder_configure: groups_per_block -1 runs one shot per group");
     groups_per_block = 0;
+  }
+  if (automatic) {
+    DeviceGuard dg(g->device);
+    Launch small{};
+    const int rc = choose_automatic(g->C, g->V, g->slots, g->vslots, d->rows, d->p.msg_type, d->max_smem, d->sm_count,
+                                    &small, &d->bulk, &d->bulk_from, "rbp_decoder_configure");
+    if (rc != RBP_OK) return rc;
+    for (int k = 0; k < 2; ++k)
+      if (kind == RBP_LAUNCH_ALL || kind == (k ? RBP_LAUNCH_LEGS : RBP_LAUNCH_PRE)) {
+        d->shape[k] = small;
+        d->automatic[k] = true;
+      }
+    return RBP_OK;
   }
   // default group size within the register budget of the kernel that runs it
   const int G = group_threads > 0 ? group_threads : default_group_threads(g->C, g->V, nshots, minb);
@@ -559,8 +628,11 @@ int rbp_decoder_configure_kind(rbp_decoder* d, int32_t kind, int32_t group_threa
   const int rc = choose_launch(g->C, g->V, g->slots, g->vslots, d->rows, d->p.msg_type, G, groups_per_block,
                                d->max_smem, d->sm_count, &lc, "rbp_decoder_configure", nshots, minb);
   if (rc != RBP_OK) return rc;
-  if (kind != RBP_LAUNCH_LEGS) d->shape[0] = lc;
-  if (kind != RBP_LAUNCH_PRE) d->shape[1] = lc;
+  for (int k = 0; k < 2; ++k)
+    if (kind == RBP_LAUNCH_ALL || kind == (k ? RBP_LAUNCH_LEGS : RBP_LAUNCH_PRE)) {
+      d->shape[k] = lc;
+      d->automatic[k] = false;
+    }
   return RBP_OK;
 }
 
@@ -687,7 +759,8 @@ int rbp_decode(rbp_decoder* d, int64_t B, const rbp_batch* in, const rbp_outputs
   DeviceGuard dg(g->device);
   if (!dg.ok) return fail(RBP_ERR_CUDA, "rbp_decode: cannot select the CUDA device");
   // a launch that skips the relay legs runs at most pre_iter iterations per shot
-  const Launch& sh = d->shape[in->skip_relay_legs ? 0 : 1];
+  const int k = in->skip_relay_legs ? 0 : 1;
+  const Launch& sh = d->automatic[k] && B >= d->bulk_from ? d->bulk : d->shape[k];
   return launch_decode(device_graph(*d), d->p, sh, d->llr.p, d->gamma_legs.p, d->alpha.p, d->strict, d->queue.p, B, in,
                        out, reinterpret_cast<cudaStream_t>(stream), "rbp_decode");
 }
@@ -1153,11 +1226,15 @@ int rbp_decode_static(int32_t C, int32_t V, int32_t E, const int32_t* chk_ptr, c
   }
   if ((rc = flush())) return rc;
 
-  int G = default_group_threads(C, V), max_smem = 0, sms = 0;
+  int max_smem = 0, sms = 0;
   RBP_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   RBP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   Launch lc{};
-  if ((rc = choose_launch(C, V, slots, vslots, rows, p->msg_type, G, 0, (size_t)max_smem, sms, &lc, who))) return rc;
+  Launch bulk{};
+  int64_t bulk_from = 0;
+  if ((rc = choose_automatic(C, V, slots, vslots, rows, p->msg_type, (size_t)max_smem, sms, &lc, &bulk, &bulk_from, who)))
+    return rc;
+  if (B >= bulk_from) lc = bulk;
   const DevGraph dgph{C, V, E, slots, rows, vslots, scratch + off_deg, reinterpret_cast<const int*>(scratch + off_ptr),
                       reinterpret_cast<const uint16_t*>(scratch + off_pos),
                       reinterpret_cast<const uint16_t*>(scratch + off_chk), cs};

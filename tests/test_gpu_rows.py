@@ -16,7 +16,7 @@ from pelagos_b200 import RelayBPDecoder
 pytestmark = pytest.mark.gpu
 
 DEV = "cuda:0"
-SHAPES = [None, (0, 1), (0, 1, 2), (0, 1, 1, 2)]
+SHAPES = [None, (0, -1), (64, 2), (0, 1), (0, 1, 2), (0, 1, 1, 2)]  # the library's choice, groups in a block, ...
 BASE = dict(pre_iter=24, num_sets=4, set_max_iter=15, gamma0=0.65, gamma_dist_interval=(-0.24, 0.66), stop_nconv=3,
             algo="relay", seed=5)
 VARIANTS = {
@@ -72,7 +72,8 @@ def _oracle(dec, syn, mix, **kw):
 def test_irregular_graphs_match_oracle(size, dtype):
     H = _graph(*size, seed=size[0])
     syn = _syndromes(H, 0.03, 48, seed=3)
-    for shape in SHAPES if size[2] <= 16 else SHAPES[:1]:
+    shapes = [s for s in SHAPES if s != (64, 2) or size[1] <= 1024]  # 64 threads own at most 1,024 variables
+    for shape in shapes if size[2] <= 16 else shapes[:2]:
         for name, kw in VARIANTS.items():
             dec = RelayBPDecoder(H, np.full(size[1], 0.03), data_type=dtype, launch=shape, **{**BASE, **kw})
             out = dec.decode(torch.from_numpy(syn).to(DEV), return_last_posterior=True)
