@@ -398,6 +398,25 @@ RBP_API int rbp_net_propose(rbp_net* n, int64_t B, const uint8_t* syn, const flo
 RBP_API int rbp_gf2_matvec(const uint8_t* x, int64_t B, int32_t N, const int32_t* row_ptr, const int32_t* cols,
                            int32_t R, uint8_t* out, void* stream);
 
+/*
+ * Result arrays of a decode in one launch (asynchronous on `stream`, device
+ * pointers; src/pelagos/decoder.py:3839-3873): weights [B] (float, or double
+ * with weights_f64 = 1; weight_fixed * 2^-32, +inf where it is INT64_MAX),
+ * valid [B] (1 where found_count >= stop_nconv), and the indices of the other
+ * shots in ascending order in unconverged [capacity B] with their number in
+ * *n_unconverged.
+ */
+RBP_API int rbp_results(const int32_t* found_count, const int64_t* weight_fixed, int64_t B, int32_t stop_nconv,
+                        void* weights, int32_t weights_f64, uint8_t* valid, int32_t* unconverged,
+                        int32_t* n_unconverged, void* stream);
+
+/*
+ * Queue order (rbp_batch.shot_order) that takes the shots without a solution
+ * (found_count <= 0) first, each part in ascending order; their number goes to
+ * *n_unsolved unless it is NULL.  One launch, asynchronous on `stream`.
+ */
+RBP_API int rbp_queue_order(const int32_t* found_count, int64_t B, int32_t* order, int32_t* n_unsolved, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

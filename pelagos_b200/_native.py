@@ -65,6 +65,8 @@ EXPORTED_SYMBOLS = (
     "rbp_net_train_step",
     "rbp_net_propose",
     "rbp_gf2_matvec",
+    "rbp_results",
+    "rbp_queue_order",
 )
 
 #: Bytes of the static scratch array rbp_decode_static uses (RBP_STATIC_SCRATCH_BYTES).
@@ -221,6 +223,10 @@ def _declare(lib):
     lib.rbp_net_propose.argtypes = [P, i64, P, P, i64, ct.c_float, ct.c_float, P, P, P, P, P]
     lib.rbp_gf2_matvec.restype = ct.c_int
     lib.rbp_gf2_matvec.argtypes = [P, i64, i32, P, P, i32, P, P]
+    lib.rbp_results.restype = ct.c_int
+    lib.rbp_results.argtypes = [P, P, i64, i32, P, i32, P, P, P, P]
+    lib.rbp_queue_order.restype = ct.c_int
+    lib.rbp_queue_order.argtypes = [P, i64, P, P, P]
     return lib
 
 

@@ -70,6 +70,31 @@ def _ptr(t: Optional[torch.Tensor]):
 #: Batches at least this large decode with the unconverged shots queued first (hard_shots_first).
 HARD_FIRST_MIN_BATCH = 1024
 
+def finish_results(found: torch.Tensor, wfix: torch.Tensor, stop_nconv: int, weights_dtype=torch.float32):
+    """(weights, valid mask, unconverged indices) of a decode's device counts and exact weights, on the
+    current device and stream; reading the number of unconverged shots synchronises the host."""
+    B, dev = int(found.shape[0]), found.device
+    weights = torch.empty(B, dtype=weights_dtype, device=dev)
+    valid = torch.empty(B, dtype=torch.bool, device=dev)
+    unconverged = torch.empty(B + 1, dtype=torch.int32, device=dev)  # their number comes after the capacity
+    f64 = 1 if weights_dtype == torch.float64 else 0
+    u = unconverged.data_ptr()
+    nat.check(nat.lib().rbp_results(found.data_ptr(), wfix.data_ptr(), B, int(stop_nconv), weights.data_ptr(), f64,
+                                    valid.data_ptr(), u, u + 4 * B, torch.cuda.current_stream(dev).cuda_stream),
+              "rbp_results")
+    return weights, valid, unconverged[:int(unconverged[B])]
+
+
+def queue_order(found: torch.Tensor, count: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Shot order with the shots that have no solution first (their number in ``count``), on the
+    current stream."""
+    order = torch.empty(found.shape[0], dtype=torch.int32, device=found.device)
+    nat.check(nat.lib().rbp_queue_order(found.data_ptr(), int(found.shape[0]), order.data_ptr(),
+                                        count.data_ptr() if count is not None else None,
+                                        torch.cuda.current_stream(found.device).cuda_stream), "rbp_queue_order")
+    return order
+
+
 class _NativeDecoder:
     """Owns one device's rbp_graph + rbp_decoder handles."""
 
@@ -669,8 +694,7 @@ class RelayBPDecoder:
             state = self._state_buffer(gpu_id, B)
             first = self._decode_on(gpu_id, syn, 0, pre, init_posterior, init_gamma, True, False, prior_llr,
                                     leg_gammas, None, state, 0, 0, light=True)
-            # stable: converged shots (key 1) keep their order after the unconverged ones (key 0)
-            order = torch.argsort((first["found_count"] > 0).to(torch.uint8), stable=True).to(torch.int32)
+            order = queue_order(first["found_count"])  # the unconverged ones, then the converged, both in order
             return self._launch_on(gpu_id, syn, 0, pre, None, None, False, return_last_posterior, prior_llr,
                                    leg_gammas, state, None, 0, 0, order=order)
 
@@ -752,17 +776,15 @@ class RelayBPDecoder:
         """The result dict of a launch's buffers (the unconverged-index list synchronises the host)."""
         found, iters, wfix = raw["found"], raw["iters"], raw["wfix"]
         with torch.cuda.device(raw["gpu_id"]):
-            has = wfix != torch.iinfo(torch.int64).max
             wdt = torch.float64 if self.dtype_str == "float64" else torch.float32
-            weights = torch.where(has, wfix.to(torch.float64) * (2.0 ** -32),
-                                  torch.full_like(wfix, 0, dtype=torch.float64) + float("inf")).to(wdt)
+            weights, valid, unconverged = finish_results(found, wfix, self.stop_nconv, wdt)
             result = {
                 "errors": raw["packed"] if self.bitpack_output else raw["errors"],
                 "weights": weights,
-                "valid_mask": found >= self.stop_nconv,
+                "valid_mask": valid,
                 "iterations": iters,
                 "found_count": found,
-                "unconverged_indices": torch.nonzero(found < self.stop_nconv).flatten().to(torch.int32),
+                "unconverged_indices": unconverged,
                 "weight_fixed": wfix,
             }
             if raw["last_post"] is not None:

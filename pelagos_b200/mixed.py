@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from . import _native as nat
-from .decoder import RelayBPDecoder, _ptr
+from .decoder import RelayBPDecoder, _ptr, finish_results
 
 
 class MixedDecoder:
@@ -123,16 +123,14 @@ class MixedDecoder:
             for d, buf in zip(self.decoders, self._bufs):
                 wfix = buf["weight_fixed"].clone()
                 found = buf["found_count"].clone()
-                has = wfix != torch.iinfo(torch.int64).max
-                weights = torch.where(has, wfix.to(torch.float64) * (2.0 ** -32),
-                                      torch.full_like(wfix, 0, dtype=torch.float64) + float("inf")).to(torch.float32)
+                weights, valid, unconverged = finish_results(found, wfix, d.stop_nconv)
                 results.append({
                     "errors": buf["errors"].clone(),
                     "weights": weights,
-                    "valid_mask": found >= d.stop_nconv,
+                    "valid_mask": valid,
                     "iterations": buf["iterations"].clone(),
                     "found_count": found,
-                    "unconverged_indices": torch.nonzero(found < d.stop_nconv).flatten().to(torch.int32),
+                    "unconverged_indices": unconverged,
                     "weight_fixed": wfix,
                 })
             return results

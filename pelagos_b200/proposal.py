@@ -35,7 +35,7 @@ import numpy as np
 import torch
 
 from . import _native as nat
-from .decoder import RelayBPDecoder, _ptr
+from .decoder import RelayBPDecoder, _ptr, finish_results, queue_order
 
 DATA_DIR = Path(__file__).resolve().parent / "data"
 
@@ -353,14 +353,12 @@ class LearnedRelayBPDecoder:
         d._native[gid].decode(B, pre_in, pre_out, stream)
         if events is not None:
             events[1].record()
-        unsolved = bf["found"] == 0
-        order = torch.argsort((~unsolved).to(torch.uint8), stable=True).to(torch.int32)  # unconverged first
+        order = queue_order(bf["found"], bf["count"])  # unconverged first
         post = bf["state"].data_ptr() + self._post_offset()  # posteriors, read from the saved states
         stride = bf["state"].shape[1] // 4
         if self.gate:
             # solved shots take the constant hi in the kernel; only unsolved rows are written
             if self.network:
-                bf["count"].copy_(unsolved.sum().to(torch.int32).view(1))
                 self.net.propose_into(B, syn, post, self.lo, self.hi, bf["gammas"], order, bf["count"],
                                       post_stride=stride)
         else:
@@ -398,9 +396,7 @@ class LearnedRelayBPDecoder:
         d._native[gid].decode(B, first_in, outs, stream)
         if events is not None:
             events[1].record()
-        unsolved = bf["found"] == 0
-        order = torch.argsort((~unsolved).to(torch.uint8), stable=True).to(torch.int32)
-        bf["count"].copy_(unsolved.sum().to(torch.int32).view(1))
+        order = queue_order(bf["found"], bf["count"])
         stride = bf["state"].shape[1]
         if self.network:
             self.net.propose_into(B, syn, bf["state"].data_ptr() + self._post_offset(), self.lo, self.hi,
@@ -436,16 +432,14 @@ class LearnedRelayBPDecoder:
         else:
             bf = self.decode_into(syndromes.to(device=self.net.device, dtype=torch.uint8).contiguous(), events)
         wfix, found = bf["wfix"].clone(), bf["found"].clone()
-        has = wfix != torch.iinfo(torch.int64).max
-        weights = torch.where(has, wfix.to(torch.float64) * (2.0 ** -32),
-                              torch.full_like(wfix, 0, dtype=torch.float64) + float("inf")).to(torch.float32)
+        weights, valid, unconverged = finish_results(found, wfix, d.stop_nconv)
         return {
             "errors": bf["errors"].clone(),
             "weights": weights,
-            "valid_mask": found >= d.stop_nconv,
+            "valid_mask": valid,
             "iterations": bf["iters"].clone(),
             "found_count": found,
-            "unconverged_indices": torch.nonzero(found < d.stop_nconv).flatten().to(torch.int32),
+            "unconverged_indices": unconverged,
             "weight_fixed": wfix,
         }
 
