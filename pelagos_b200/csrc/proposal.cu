@@ -163,7 +163,7 @@ __global__ void feat_var_kernel(NetGraph g, long long B, const uint8_t* syn, con
 // Arrays are stored in 16-byte columns ([chunk][row]), so a warp's accesses are
 // contiguous.  With one thread per output element, each layer re-reading and re-writing
 // the node states (245 MB each for 1,024 shots of the 936 x 2,592 graph), a step of
-// 1,024 shots took 9.71 ms; now 2.08.
+// 1,024 shots took 9.71 ms; now 1.82.
 
 // Gradients are summed in three steps: fp32 within a block (over its rows), one partial sum
 // per block in memory, and the blocks' sums in double.  With an atomic add per block the
@@ -171,6 +171,13 @@ __global__ void feat_var_kernel(NetGraph g, long long B, const uint8_t* syn, con
 constexpr int GRAD_BLOCKS = 148 * 4;               // at most so many blocks add to a parameter
 constexpr int GRAD_STRIDE = (N_PARAMS + 1 + 3) / 4 * 4;  // the loss comes after the parameters
 constexpr int RT = 128;       // threads (rows) of a row kernel's tile
+// Rows per thread and resident blocks per SM of the row kernels: each weight read from shared
+// memory serves that many rows.  us per launch at 958,464 rows, one row at 6 (forward) and 4
+// blocks / two rows at 4 and 2: forward 108, 204, 217 / 86, 179, 192 (four rows: 108, 253, 266);
+// backward stages 0, 1, 2: 305, 250, 190 / 274, 241, 234.
+constexpr int FR = 2, FB = 4;
+__host__ __device__ constexpr int back_rows(int stage) { return stage == 2 ? 1 : 2; }
+__host__ __device__ constexpr int back_blocks(int stage) { return stage == 2 ? 4 : 2; }
 constexpr int SY = NH + 4;    // padded shared-memory rows of the gradient tiles
 constexpr int SX = ND + 4;
 
@@ -223,41 +230,52 @@ __device__ __forceinline__ void store16(float4* p, size_t n, size_t i, const flo
   for (int q = 0; q < 4; ++q) p[q * n + i] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
 }
 
-// acc + sum_k f[k] w[k], k ascending, w 16 floats in shared memory
-__device__ __forceinline__ float dot16(const float (&f)[16], const float* w, float acc) {
+// acc[r] + sum_k f[r][k] w[k], k ascending, w 16 floats in shared memory
+template <int R>
+__device__ __forceinline__ void dot16(const float (&f)[R][16], const float* w, float (&acc)[R]) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const float4 v = *reinterpret_cast<const float4*>(w + 4 * q);
-    acc = fmaf(f[4 * q], v.x, acc);
-    acc = fmaf(f[4 * q + 1], v.y, acc);
-    acc = fmaf(f[4 * q + 2], v.z, acc);
-    acc = fmaf(f[4 * q + 3], v.w, acc);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      acc[r] = fmaf(f[r][4 * q], v.x, acc[r]);
+      acc[r] = fmaf(f[r][4 * q + 1], v.y, acc[r]);
+      acc[r] = fmaf(f[r][4 * q + 2], v.z, acc[r]);
+      acc[r] = fmaf(f[r][4 * q + 3], v.w, acc[r]);
+    }
   }
-  return acc;
 }
 
-// acc[k] += y w[k]
-__device__ __forceinline__ void axpy16(float y, const float* w, float (&acc)[16]) {
+// acc[r][k] += y[r] w[k]
+template <int R>
+__device__ __forceinline__ void axpy16(const float (&y)[R], const float* w, float (&acc)[R][16]) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const float4 v = *reinterpret_cast<const float4*>(w + 4 * q);
-    acc[4 * q] = fmaf(y, v.x, acc[4 * q]);
-    acc[4 * q + 1] = fmaf(y, v.y, acc[4 * q + 1]);
-    acc[4 * q + 2] = fmaf(y, v.z, acc[4 * q + 2]);
-    acc[4 * q + 3] = fmaf(y, v.w, acc[4 * q + 3]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      acc[r][4 * q] = fmaf(y[r], v.x, acc[r][4 * q]);
+      acc[r][4 * q + 1] = fmaf(y[r], v.y, acc[r][4 * q + 1]);
+      acc[r][4 * q + 2] = fmaf(y[r], v.z, acc[r][4 * q + 2]);
+      acc[r][4 * q + 3] = fmaf(y[r], v.w, acc[r][4 * q + 3]);
+    }
   }
 }
 
 // q0_j = E_j . x^
-__device__ __forceinline__ float embed(const float (&x)[8], const float* e) {
+template <int R>
+__device__ __forceinline__ void embed(const float (&x)[R][8], const float* e, float (&acc)[R]) {
   const float4 u = *reinterpret_cast<const float4*>(e);
   const float2 v = *reinterpret_cast<const float2*>(e + 4);
-  float acc = fmaf(x[0], u.x, 0.f);
-  acc = fmaf(x[1], u.y, acc);
-  acc = fmaf(x[2], u.z, acc);
-  acc = fmaf(x[3], u.w, acc);
-  acc = fmaf(x[4], v.x, acc);
-  return fmaf(x[5], v.y, acc);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    acc[r] = fmaf(x[r][0], u.x, 0.f);
+    acc[r] = fmaf(x[r][1], u.y, acc[r]);
+    acc[r] = fmaf(x[r][2], u.z, acc[r]);
+    acc[r] = fmaf(x[r][3], u.w, acc[r]);
+    acc[r] = fmaf(x[r][4], v.x, acc[r]);
+    acc[r] = fmaf(x[r][5], v.y, acc[r]);
+  }
 }
 
 // Weights as fp32 in shared memory: E as [64][8], W (given [16][64]) transposed to [64][16].
@@ -273,8 +291,9 @@ __device__ __forceinline__ void stage(const bf16* w, int n, float* s) {
 
 // Forward of a row up to its next message (STAGE 1: x^ -> m1; 2: a1 -> m2) or readout (3: a2 -> o).
 template <int STAGE>
-__global__ void __launch_bounds__(RT) rows_forward_kernel(NetGraph g, unsigned nc, unsigned nv, NetWork w,
-                                                          const bf16* theta, const uint8_t* syn, const float* lmean) {
+__global__ void __launch_bounds__(RT, FB) rows_forward_kernel(NetGraph g, unsigned nc, unsigned nv, NetWork w,
+                                                              const bf16* theta, const uint8_t* syn,
+                                                              const float* lmean) {
   __shared__ __align__(16) float sE[NH * 8], sW[NH * ND], sU1[NH * ND], sU2[STAGE == 3 ? NH * ND : 4];
   __shared__ float sb1[NH], sb2[NH], sO[NH];
   __shared__ __align__(16) float sG[NTY * SX];
@@ -293,94 +312,108 @@ __global__ void __launch_bounds__(RT) rows_forward_kernel(NetGraph g, unsigned n
     stage(theta + P_O, NH, sO);
   }
   __syncthreads();
-  for (unsigned row = blockIdx.x * RT + threadIdx.x; row < nc; row += gridDim.x * RT) {
-    const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
-    const int e0 = g.chk_ptr[c], e1 = g.chk_ptr[c + 1];
-    const size_t v0 = (size_t)b * g.V;
-    float x[8];
-    if constexpr (STAGE == 1) {
-      float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-      for (int e = e0; e < e1; ++e) {
-        const float4 f = __ldg(reinterpret_cast<const float4*>(w.z) + v0 + g.chk_var[e]);
-        s0 += f.x;
-        s1 += f.y;
-        s2 += f.z;
-      }
-      const float deg = (float)max(e1 - e0, 1);
-      x[0] = (float)(syn[row] & 1);
-      x[1] = s0 / deg;
-      x[2] = s1 / deg;
-      x[3] = s2 / deg;
-      x[4] = lmean[c];
-      x[5] = 1.f;
-      x[6] = x[7] = 0.f;
-      const uint4 q = pack8(x);
-      w.x[row] = q;
-      unpack8(q, x);
-    } else {
-      unpack8(__ldg(w.x + row), x);
-    }
-    float a[16];
-    float al[16];  // layer 1's aggregates in stage 3
-    if constexpr (STAGE >= 2) {
-      // a_c = sum_{v in N(c)} G[t_v] (n_v - m_c)
-      const uint4* n = STAGE == 2 ? w.n1 : w.n2;
-      float mc[16];
-      load16(STAGE == 2 ? w.m1 : w.m2, nc, row, mc);
+  for (unsigned r0 = blockIdx.x * (RT * FR) + threadIdx.x; r0 < nc; r0 += gridDim.x * (RT * FR)) {
+    float x[FR][8], a[FR][16], al[FR][16];  // al: layer 1's aggregates in stage 3
 #pragma unroll
-      for (int k = 0; k < 16; ++k) a[k] = 0.f;
-      for (int e = e0; e < e1; ++e) {
-        const size_t v = v0 + g.chk_var[e];
-        float nf[16];
-        load16(n, nv, v, nf);
-        const float* gt = sG + __ldg(w.ty + v) * SX;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float4 t = *reinterpret_cast<const float4*>(gt + 4 * q);
-          a[4 * q] = fmaf(t.x, nf[4 * q] - mc[4 * q], a[4 * q]);
-          a[4 * q + 1] = fmaf(t.y, nf[4 * q + 1] - mc[4 * q + 1], a[4 * q + 1]);
-          a[4 * q + 2] = fmaf(t.z, nf[4 * q + 2] - mc[4 * q + 2], a[4 * q + 2]);
-          a[4 * q + 3] = fmaf(t.w, nf[4 * q + 3] - mc[4 * q + 3], a[4 * q + 3]);
+    for (int i = 0; i < FR; ++i) {
+      const unsigned row = min(r0 + i * RT, nc - 1);  // past the end: the last row once more, not stored
+      const bool in = r0 + i * RT < nc;
+      const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
+      const int e0 = g.chk_ptr[c], e1 = g.chk_ptr[c + 1];
+      const size_t v0 = (size_t)b * g.V;
+      if constexpr (STAGE == 1) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+        for (int e = e0; e < e1; ++e) {
+          const float4 f = __ldg(reinterpret_cast<const float4*>(w.z) + v0 + g.chk_var[e]);
+          s0 += f.x;
+          s1 += f.y;
+          s2 += f.z;
         }
+        const float deg = (float)max(e1 - e0, 1);
+        const float xi[8] = {(float)(syn[row] & 1), s0 / deg, s1 / deg, s2 / deg, lmean[c], 1.f, 0.f, 0.f};
+        const uint4 q = pack8(xi);
+        if (in) w.x[row] = q;
+        unpack8(q, x[i]);
+      } else {
+        unpack8(__ldg(w.x + row), x[i]);
       }
-      store16(STAGE == 2 ? w.a1 : w.a2, nc, row, a);
+      if constexpr (STAGE >= 2) {
+        // a_c = sum_{v in N(c)} G[t_v] (n_v - m_c)
+        const uint4* n = STAGE == 2 ? w.n1 : w.n2;
+        float mc[16];
+        load16(STAGE == 2 ? w.m1 : w.m2, nc, row, mc);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) a[k] = rbf(a[k]);  // the layer's input
-      if constexpr (STAGE == 3) load16(w.a1, nc, row, al);
+        for (int k = 0; k < 16; ++k) a[i][k] = 0.f;
+        for (int e = e0; e < e1; ++e) {
+          const size_t v = v0 + g.chk_var[e];
+          float nf[16];
+          load16(n, nv, v, nf);
+          const float* gt = sG + __ldg(w.ty + v) * SX;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 t = *reinterpret_cast<const float4*>(gt + 4 * q);
+            a[i][4 * q] = fmaf(t.x, nf[4 * q] - mc[4 * q], a[i][4 * q]);
+            a[i][4 * q + 1] = fmaf(t.y, nf[4 * q + 1] - mc[4 * q + 1], a[i][4 * q + 1]);
+            a[i][4 * q + 2] = fmaf(t.z, nf[4 * q + 2] - mc[4 * q + 2], a[i][4 * q + 2]);
+            a[i][4 * q + 3] = fmaf(t.w, nf[4 * q + 3] - mc[4 * q + 3], a[i][4 * q + 3]);
+          }
+        }
+        if (in) store16(STAGE == 2 ? w.a1 : w.a2, nc, row, a[i]);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) a[i][k] = rbf(a[i][k]);  // the layer's input
+        if constexpr (STAGE == 3) load16(w.a1, nc, row, al[i]);
+      }
     }
-    float m[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) m[k] = 0.f;
-    float o = 0.f;
-    unsigned long long mask = 0ull;
+    float m[FR][16] = {}, o[FR] = {};
+    unsigned long long mask[FR] = {};
 #pragma unroll 1
     for (int ch = 0; ch < NH / 8; ++ch) {
-      float gv[8];
+      float gv[FR][8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int j = ch * 8 + i;
-        float q = embed(x, sE + j * 8);
-        if constexpr (STAGE == 2) q = dot16(a, sU1 + j * ND, 0.f) + sb1[j] + fmaxf(q, 0.f);
-        if constexpr (STAGE == 3) {
-          q = dot16(al, sU1 + j * ND, 0.f) + sb1[j] + fmaxf(q, 0.f);
-          q = dot16(a, sU2 + j * ND, 0.f) + sb2[j] + fmaxf(q, 0.f);
+      for (int k = 0; k < 8; ++k) {
+        const int j = ch * 8 + k;
+        float q[FR], y[FR];
+        embed(x, sE + j * 8, q);
+        if constexpr (STAGE >= 2) {
+          float u[FR] = {};
+          if constexpr (STAGE == 2) dot16(a, sU1 + j * ND, u);
+          else dot16(al, sU1 + j * ND, u);
+#pragma unroll
+          for (int i = 0; i < FR; ++i) q[i] = u[i] + sb1[j] + fmaxf(q[i], 0.f);
         }
-        if (q > 0.f) mask |= 1ull << j;
-        gv[i] = rbf(fmaxf(q, 0.f));
-        if constexpr (STAGE < 3) axpy16(gv[i], sW + j * ND, m);
-        else o = fmaf(gv[i], sO[j], o);
+        if constexpr (STAGE == 3) {
+          float u[FR] = {};
+          dot16(a, sU2 + j * ND, u);
+#pragma unroll
+          for (int i = 0; i < FR; ++i) q[i] = u[i] + sb2[j] + fmaxf(q[i], 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < FR; ++i) {
+          if (q[i] > 0.f) mask[i] |= 1ull << j;
+          gv[i][k] = y[i] = rbf(fmaxf(q[i], 0.f));
+          if constexpr (STAGE == 3) o[i] = fmaf(y[i], sO[j], o[i]);
+        }
+        if constexpr (STAGE < 3) axpy16(y, sW + j * ND, m);
       }
-      if constexpr (STAGE == 2) w.g1[(size_t)ch * nc + row] = pack8(gv);
-      if constexpr (STAGE == 3) w.g2[(size_t)ch * nc + row] = pack8(gv);
+      if constexpr (STAGE >= 2) {
+#pragma unroll
+        for (int i = 0; i < FR; ++i)
+          if (r0 + i * RT < nc) (STAGE == 2 ? w.g1 : w.g2)[(size_t)ch * nc + r0 + i * RT] = pack8(gv[i]);
+      }
     }
-    if constexpr (STAGE == 1) store16(w.m1, nc, row, m);
-    if constexpr (STAGE == 2) {
-      store16(w.m2, nc, row, m);
-      w.k1[row] = mask;
-    }
-    if constexpr (STAGE == 3) {
-      w.o[row] = o;
-      w.k2[row] = mask;
+#pragma unroll
+    for (int i = 0; i < FR; ++i) {
+      const unsigned row = r0 + i * RT;
+      if (row >= nc) break;
+      if constexpr (STAGE == 1) store16(w.m1, nc, row, m[i]);
+      if constexpr (STAGE == 2) {
+        store16(w.m2, nc, row, m[i]);
+        w.k1[row] = mask[i];
+      }
+      if constexpr (STAGE == 3) {
+        w.o[row] = o[i];
+        w.k2[row] = mask[i];
+      }
     }
   }
 }
@@ -488,43 +521,50 @@ __global__ void __launch_bounds__(512) dm_kernel(NetGraph g, unsigned nc, unsign
   }
 }
 
-// acc[i][k] += sum over the tile's rows of y[2 jp + i] x[4 kq + k]: a thread's 2 x 4 block of the
-// outer products summed over RT rows, 8 fmas per two shared-memory loads.
-__device__ __forceinline__ void outer_sum(const float* sy, const float* sx, int jp, int kq, float (&acc)[2][4]) {
-#pragma unroll 8
-  for (int r = 0; r < RT; ++r) {
-    const float2 y = *reinterpret_cast<const float2*>(sy + r * SY + 2 * jp);
+// acc[i][k] += sum over a warp's tile of y[j(i)] x[4 kq + k], j(i) = 4 jq + i, then 32 + 4 jq + i - 4: a lane's
+// 8 x 4 block of the 64 x 16 outer products, 32 fmas per three 16-byte shared-memory loads.
+template <int WR>
+__device__ __forceinline__ void outer_sum(const float* sy, const float* sx, int jq, int kq, float (&acc)[8][4]) {
+#pragma unroll 4
+  for (int r = 0; r < WR; ++r) {
+    const float4 y0 = *reinterpret_cast<const float4*>(sy + r * SY + 4 * jq);
+    const float4 y1 = *reinterpret_cast<const float4*>(sy + r * SY + 32 + 4 * jq);
     const float4 x = *reinterpret_cast<const float4*>(sx + r * SX + 4 * kq);
-    acc[0][0] = fmaf(y.x, x.x, acc[0][0]);
-    acc[0][1] = fmaf(y.x, x.y, acc[0][1]);
-    acc[0][2] = fmaf(y.x, x.z, acc[0][2]);
-    acc[0][3] = fmaf(y.x, x.w, acc[0][3]);
-    acc[1][0] = fmaf(y.y, x.x, acc[1][0]);
-    acc[1][1] = fmaf(y.y, x.y, acc[1][1]);
-    acc[1][2] = fmaf(y.y, x.z, acc[1][2]);
-    acc[1][3] = fmaf(y.y, x.w, acc[1][3]);
+    const float y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      acc[i][0] = fmaf(y[i], x.x, acc[i][0]);
+      acc[i][1] = fmaf(y[i], x.y, acc[i][1]);
+      acc[i][2] = fmaf(y[i], x.z, acc[i][2]);
+      acc[i][3] = fmaf(y[i], x.w, acc[i][3]);
+    }
   }
 }
 
 // Backward of a row from the readout (STAGE 2) or from dm2 (1) to the aggregates' gradients da,
-// or from dm1 to the inputs (0), and the weight gradients of that stretch: per tile of RT rows
-// each 64-wide vector (dq, then the layer's input g) is laid in shared memory next to the
-// 16-wide one it multiplies, and a thread adds up its 2 x 4 block of the outer products.
+// or from dm1 to the inputs (0), and the weight gradients of that stretch: per warp and
+// tile of rows each 64-wide vector (dq, then the layer's input g) is laid in shared memory next
+// to the 16-wide one it multiplies, and a lane adds up its 8 x 4 block of the outer products
+// over the warp's own rows, without a block barrier until the warps' sums are added up at the
+// end.  Shared-memory loads bound these kernels more than the fmas: with a tile per block and
+// 2 x 4 blocks (two loads per 8 fmas) the stages took 339, 307 and 255 us, now 274, 241 and 190.
 //   dq2_j = dout O_j [q2_j > 0],  dq1 = (dq2 + W2^T dm2) [q1 > 0],  dq0 = (dq1 + W1^T dm1) [q0 > 0]
 //   2: dO += dout g2, dU2 += dq2 a2^T, db2 += dq2, da = U2^T dq2
 //   1: dW2 += dm2 g1^T, dU1 += dq1 a1^T, db1 += dq1, da = U1^T dq1
 //   0: dW1 += dm1 g0^T, dE += dq0 x^T
 template <int STAGE>
-__global__ void __launch_bounds__(RT) rows_backward_kernel(NetGraph g, unsigned nc, NetWork w, const bf16* theta,
-                                                           const float* dr, float* grad) {
+__global__ void __launch_bounds__(RT, back_blocks(STAGE)) rows_backward_kernel(NetGraph g, unsigned nc, NetWork w, const bf16* theta,
+                                                               const float* dr, float* grad) {
+  constexpr int BR = back_rows(STAGE), WR = 32 * BR;  // rows of a thread, of a warp's tile
   extern __shared__ __align__(16) float sm[];
-  float* sy = sm;                  // [RT][SY]
-  float* sx = sy + RT * SY;        // [RT][SX]
-  float* sO = sx + RT * SX;        // [64]
-  float* sW2 = sO + NH;            // [64][16] transposed (stages 1, 0)
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, jq = lane >> 2, kq = lane & 3;
+  float* sy = sm + warp * (WR * (SY + SX));      // this warp's [WR][SY]
+  float* sx = sy + WR * SY;                      // [WR][SX]
+  float* sO = sm + RT / 32 * (WR * (SY + SX));   // [64]
+  float* sW2 = sO + NH;                          // [64][16] transposed (stages 1, 0)
   float* sU = sW2 + (STAGE == 2 ? 0 : NH * ND);  // [64][16]: U2 or U1 (stages 2, 1)
-  float* sW1 = sU;                 // [64][16] transposed (stage 0)
-  float* sE = sW1 + NH * ND;       // [64][8] (stage 0)
+  float* sW1 = sU;                               // [64][16] transposed (stage 0)
+  float* sE = sW1 + NH * ND;                     // [64][8] (stage 0)
   stage(theta + P_O, NH, sO);
   if (STAGE == 2) stage(theta + P_U2, NH * ND, sU);
   if (STAGE == 1) stage(theta + P_U1, NH * ND, sU);
@@ -533,138 +573,192 @@ __global__ void __launch_bounds__(RT) rows_backward_kernel(NetGraph g, unsigned 
     stage_t(theta + P_W1, sW1);
     stage_e(theta, sE);
   }
-  const int t = threadIdx.x, jp = t >> 2, kq = t & 3;
-  float acc_y[2][4] = {}, acc_g[2][4] = {}, acc_b[2] = {};
-  for (unsigned r0 = blockIdx.x * RT; r0 < nc; r0 += gridDim.x * RT) {
-    const unsigned row = r0 + t;
-    const bool in = row < nc;
-    float da[16], dm2[16], dm1[16], x[8];
+  __syncthreads();
+  float acc_y[8][4] = {}, acc_g[8][4] = {}, acc_b[2] = {}, acc_o[2] = {};
+  const unsigned nt = (nc + WR - 1) / WR;  // tiles of a warp's rows
+  for (unsigned tile = blockIdx.x * (RT / 32) + warp; tile < nt; tile += gridDim.x * (RT / 32)) {
+    float da[BR][16] = {}, dm2[BR][16] = {}, dm1[BR][16] = {}, x[BR][8] = {}, dout[BR] = {};
+    unsigned long long k2[BR] = {}, k1[BR] = {};
+    __syncwarp();  // the last tile's sums are done
 #pragma unroll
-    for (int k = 0; k < 16; ++k) da[k] = dm2[k] = dm1[k] = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = 0.f;
-    float dout = 0.f;
-    unsigned long long k2 = 0ull, k1 = 0ull;
-    float* myx = sx + t * SX;
-    __syncthreads();  // the last tile's sums are done (first tile: the weights are staged)
-    if (in) {
-      k2 = w.k2[row];
-      if constexpr (STAGE == 2) {
-        const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
-        for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
-          const int v = g.chk_var[e];
-          dout += __ldg(dr + (size_t)b * g.V + v) / (float)max(g.var_ptr[v + 1] - g.var_ptr[v], 1);
+    for (int i = 0; i < BR; ++i) {
+      const unsigned row = tile * WR + i * 32 + lane;
+      const bool in = row < nc;
+      float* myx = sx + (i * 32 + lane) * SX;
+      if (in) {
+        k2[i] = w.k2[row];
+        if constexpr (STAGE == 2) {
+          const unsigned b = row / (unsigned)g.C, c = row - b * (unsigned)g.C;
+          for (int e = g.chk_ptr[c]; e < g.chk_ptr[c + 1]; ++e) {
+            const int v = g.chk_var[e];
+            dout[i] += __ldg(dr + (size_t)b * g.V + v) / (float)max(g.var_ptr[v + 1] - g.var_ptr[v], 1);
+          }
+          w.dout[row] = dout[i];
+        } else {
+          dout[i] = w.dout[row];
+          k1[i] = w.k1[row];
+          load16(w.dm2, nc, row, dm2[i]);
         }
-        w.dout[row] = dout;
-      } else {
-        dout = w.dout[row];
-        k1 = w.k1[row];
-        load16(w.dm2, nc, row, dm2);
+        if constexpr (STAGE == 0) {
+          load16(w.dm1, nc, row, dm1[i]);
+          unpack8(__ldg(w.x + row), x[i]);
+        }
       }
-      if constexpr (STAGE == 0) {
-        load16(w.dm1, nc, row, dm1);
-        unpack8(__ldg(w.x + row), x);
-      }
-    }
-    // the 16-wide factor of dq: a2, a1 or x^
-    if constexpr (STAGE == 0) {
-#pragma unroll
-      for (int k = 0; k < 16; ++k) myx[k] = k < 8 ? x[k & 7] : 0.f;
-    } else {
+      // the 16-wide factor of dq: a2, a1 or x^
       float a[16] = {};
-      if (in) load16(STAGE == 2 ? w.a2 : w.a1, nc, row, a);
+      if constexpr (STAGE == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a[k] = x[i][k];
+      } else if (in) {
+        load16(STAGE == 2 ? w.a2 : w.a1, nc, row, a);
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
         *reinterpret_cast<float4*>(myx + 4 * q) = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
     }
 #pragma unroll 1
     for (int j0 = 0; j0 < NH; j0 += 4) {
-      float dq[4];
+      float dq[BR][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int j = j0 + i;
-        float d = (k2 >> j) & 1ull ? dout * sO[j] : 0.f;
-        if constexpr (STAGE <= 1) d = (k1 >> j) & 1ull ? d + dot16(dm2, sW2 + j * ND, 0.f) : 0.f;
+      for (int k = 0; k < 4; ++k) {
+        const int j = j0 + k;
+        float d[BR], u[BR] = {};
+#pragma unroll
+        for (int i = 0; i < BR; ++i) d[i] = (k2[i] >> j) & 1ull ? dout[i] * sO[j] : 0.f;
+        if constexpr (STAGE <= 1) {
+          dot16(dm2, sW2 + j * ND, u);
+#pragma unroll
+          for (int i = 0; i < BR; ++i) d[i] = (k1[i] >> j) & 1ull ? d[i] + u[i] : 0.f;
+        }
         if constexpr (STAGE == 0) {
-          d += dot16(dm1, sW1 + j * ND, 0.f);
-          if (!(embed(x, sE + j * 8) > 0.f)) d = 0.f;
+          float u1[BR] = {}, q0[BR];
+          dot16(dm1, sW1 + j * ND, u1);
+          embed(x, sE + j * 8, q0);
+#pragma unroll
+          for (int i = 0; i < BR; ++i) d[i] = q0[i] > 0.f ? d[i] + u1[i] : 0.f;
         } else {
           axpy16(d, sU + j * ND, da);
         }
-        dq[i] = d;
+#pragma unroll
+        for (int i = 0; i < BR; ++i) dq[i][k] = d[i];
       }
-      *reinterpret_cast<float4*>(sy + t * SY + j0) = make_float4(dq[0], dq[1], dq[2], dq[3]);
+#pragma unroll
+      for (int i = 0; i < BR; ++i)
+        *reinterpret_cast<float4*>(sy + (i * 32 + lane) * SY + j0) =
+            make_float4(dq[i][0], dq[i][1], dq[i][2], dq[i][3]);
     }
     if constexpr (STAGE >= 1) {
-      if (in) store16(w.da, nc, row, da);
-    }
-    __syncthreads();
-    if (STAGE > 0 || kq < 2) outer_sum(sy, sx, jp, kq, acc_y);
-    if constexpr (STAGE >= 1) {  // biases: a quarter of the rows per kq
-#pragma unroll 8
-      for (int r = kq; r < RT; r += 4) {
-        const float2 y = *reinterpret_cast<const float2*>(sy + r * SY + 2 * jp);
-        acc_b[0] += y.x;
-        acc_b[1] += y.y;
+#pragma unroll
+      for (int i = 0; i < BR; ++i) {
+        const unsigned row = tile * WR + i * 32 + lane;
+        if (row < nc) store16(w.da, nc, row, da[i]);
       }
     }
-    __syncthreads();
+    __syncwarp();
+    outer_sum<WR>(sy, sx, jq, kq, acc_y);
+    if constexpr (STAGE >= 1) {  // biases: lane and lane + 32
+#pragma unroll 8
+      for (int r = 0; r < WR; ++r) {
+        acc_b[0] += sy[r * SY + lane];
+        acc_b[1] += sy[r * SY + 32 + lane];
+      }
+    }
+    __syncwarp();
     // the layer's input g and its factor: dout, dm2 or dm1
-#pragma unroll 1
-    for (int ch = 0; ch < NH / 8; ++ch) {
-      float gv[8] = {};
-      if constexpr (STAGE == 0) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) gv[i] = in ? rbf(fmaxf(embed(x, sE + (ch * 8 + i) * 8), 0.f)) : 0.f;
-      } else if (in) {
-        unpack8(__ldg((STAGE == 2 ? w.g2 : w.g1) + (size_t)ch * nc + row), gv);
+    for (int i = 0; i < BR; ++i) {
+      const unsigned row = tile * WR + i * 32 + lane;
+      const bool in = row < nc;
+      float* y = sy + (i * 32 + lane) * SY;
+      float* myx = sx + (i * 32 + lane) * SX;
+      if constexpr (STAGE != 0) {
+#pragma unroll
+        for (int ch = 0; ch < NH / 8; ++ch) {
+          float gv[8] = {};
+          if (in) unpack8(__ldg((STAGE == 2 ? w.g2 : w.g1) + (size_t)ch * nc + row), gv);
+          *reinterpret_cast<float4*>(y + ch * 8) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+          *reinterpret_cast<float4*>(y + ch * 8 + 4) = make_float4(gv[4], gv[5], gv[6], gv[7]);
+        }
       }
-      float* y = sy + t * SY + ch * 8;
-      *reinterpret_cast<float4*>(y) = make_float4(gv[0], gv[1], gv[2], gv[3]);
-      *reinterpret_cast<float4*>(y + 4) = make_float4(gv[4], gv[5], gv[6], gv[7]);
-    }
-    if constexpr (STAGE == 2) {
-      myx[0] = dout;
-    } else {
+      if constexpr (STAGE == 2) {
+        myx[0] = dout[i];
+      } else {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) myx[k] = STAGE == 1 ? dm2[k] : dm1[k];
+        for (int q = 0; q < 4; ++q) {
+          const float* f = (STAGE == 1 ? dm2[i] : dm1[i]) + 4 * q;
+          *reinterpret_cast<float4*>(myx + 4 * q) = make_float4(f[0], f[1], f[2], f[3]);
+        }
+      }
     }
-    __syncthreads();
+    if constexpr (STAGE == 0) {
+#pragma unroll 1
+      for (int j0 = 0; j0 < NH; j0 += 4) {
+        float gv[BR][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float q0[BR];
+          embed(x, sE + (j0 + k) * 8, q0);
+#pragma unroll
+          for (int i = 0; i < BR; ++i) gv[i][k] = rbf(fmaxf(q0[i], 0.f));
+        }
+#pragma unroll
+        for (int i = 0; i < BR; ++i)
+          *reinterpret_cast<float4*>(sy + (i * 32 + lane) * SY + j0) =
+              make_float4(gv[i][0], gv[i][1], gv[i][2], gv[i][3]);
+      }
+    }
+    __syncwarp();
     if constexpr (STAGE == 2) {
 #pragma unroll 8
-      for (int r = kq; r < RT; r += 4) {
-        const float2 y = *reinterpret_cast<const float2*>(sy + r * SY + 2 * jp);
+      for (int r = 0; r < WR; ++r) {
         const float d = sx[r * SX];
-        acc_g[0][0] = fmaf(d, y.x, acc_g[0][0]);
-        acc_g[1][0] = fmaf(d, y.y, acc_g[1][0]);
+        acc_o[0] = fmaf(d, sy[r * SY + lane], acc_o[0]);
+        acc_o[1] = fmaf(d, sy[r * SY + 32 + lane], acc_o[1]);
       }
     } else {
-      outer_sum(sy, sx, jp, kq, acc_g);
+      outer_sum<WR>(sy, sx, jq, kq, acc_g);
     }
   }
+  // the warps' sums, one after another in shared memory
+  __syncthreads();
+  float* red = sm;  // [4][1024] a warp's outer products as [j][k]
   float* out = grad + (size_t)blockIdx.x * GRAD_STRIDE;
+  static_assert(RT / 32 * NH * ND <= RT / 32 * WR * (SY + SX), "the warps' sums fit their tiles");
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int j = 2 * jp + i;
-    // biases and dO: the four kq threads of a channel pair hold a quarter of the rows each
-    float q = acc_b[i], o = acc_g[i][0];
+  for (int pass = 0; pass < 2; ++pass) {
+    if (STAGE == 2 && pass == 1) break;
 #pragma unroll
-    for (int m = 1; m < 4; m <<= 1) {
-      q += __shfl_xor_sync(0xffffffffu, q, m);
-      o += __shfl_xor_sync(0xffffffffu, o, m);
+    for (int i = 0; i < 8; ++i) {
+      const float* f = pass ? acc_g[i] : acc_y[i];
+      const int j = 4 * jq + (i < 4 ? i : 28 + i);
+      *reinterpret_cast<float4*>(red + (warp * NH + j) * ND + 4 * kq) = make_float4(f[0], f[1], f[2], f[3]);
     }
-    if (STAGE >= 1 && kq == 0) out[(STAGE == 2 ? P_B2 : P_B1) + j] = q;
-    if (STAGE == 2 && kq == 0) out[P_O + j] = o;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if constexpr (STAGE >= 1) out[(STAGE == 2 ? P_U2 : P_U1) + j * ND + 4 * kq + k] = acc_y[i][k];
-      else if (4 * kq + k < NX) out[P_E + j * NX + 4 * kq + k] = acc_y[i][k];
-      if constexpr (STAGE <= 1) out[(STAGE == 1 ? P_W2 : P_W1) + (4 * kq + k) * NH + j] = acc_g[i][k];
+    __syncthreads();
+    for (int i = t; i < NH * ND; i += RT) {
+      float q = 0.f;
+      for (int k = 0; k < RT / 32; ++k) q += red[k * NH * ND + i];
+      const int j = i / ND, k = i % ND;
+      if (pass) out[(STAGE == 1 ? P_W2 : P_W1) + k * NH + j] = q;
+      else if (STAGE >= 1) out[(STAGE == 2 ? P_U2 : P_U1) + i] = q;
+      else if (k < NX) out[P_E + j * NX + k] = q;
+    }
+    __syncthreads();
+  }
+  if constexpr (STAGE >= 1) {
+    red[(warp * 2) * NH + lane] = acc_b[0];
+    red[(warp * 2) * NH + 32 + lane] = acc_b[1];
+    red[(warp * 2 + 1) * NH + lane] = acc_o[0];
+    red[(warp * 2 + 1) * NH + 32 + lane] = acc_o[1];
+    __syncthreads();
+    if (t < (STAGE == 2 ? 2 : 1) * NH) {
+      float q = 0.f;
+      for (int k = 0; k < RT / 32; ++k) q += red[k * 2 * NH + t];
+      out[t < NH ? (STAGE == 2 ? P_B2 : P_B1) + t : P_O + t - NH] = q;
     }
   }
 }
 constexpr int rows_backward_smem(int stage) {
-  return (RT * SY + RT * SX + NH + (stage == 2 ? 1 : 2) * NH * ND + (stage == 0 ? NH * 8 : 0)) * 4;
+  return (RT * back_rows(stage) * (SY + SX) + NH + (stage == 2 ? 1 : 2) * NH * ND + (stage == 0 ? NH * 8 : 0)) * 4;
 }
 
 // ------------------------------------------------------------------ readout and loss (training path)
@@ -714,13 +808,14 @@ __global__ void __launch_bounds__(256) readout_kernel(NetGraph g, long long B, c
 }
 
 // The blocks' partial sums of each parameter (and of the loss), added in double: 8 warps share
-// 32 parameters.  rows / gates / vars: blocks of the kernels behind a parameter.
-__global__ void __launch_bounds__(256) grad_sum_kernel(const float* partial, int rows, int gates, int vars, float* grad,
-                                                       float* loss) {
+// 32 parameters.  rows / last / gates / vars: blocks of the kernels behind a parameter (last: the
+// second layer's update and readout).
+__global__ void __launch_bounds__(256) grad_sum_kernel(const float* partial, int rows, int last, int gates, int vars,
+                                                       float* grad, float* loss) {
   __shared__ double part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
   const bool gate = (p >= P_G1 && p < P_U1) || (p >= P_G2 && p < P_U2);
-  const int n = p > N_PARAMS ? 0 : (gate ? gates : (p >= P_OZ ? vars : rows));
+  const int n = p > N_PARAMS ? 0 : (gate ? gates : (p >= P_OZ ? vars : (p >= P_U2 ? last : rows)));
   double s = 0.0;
 #pragma unroll 4
   for (int k = warp; k < n; k += 8) s += (double)partial[(size_t)k * GRAD_STRIDE + p];
@@ -1455,7 +1550,7 @@ struct rbp_net {
     const NetWork& w = ws;
     const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
     // weights are staged once per block: the resident blocks loop over their rows
-    const unsigned rows = std::min<unsigned>((nc + RT - 1) / RT, 148 * 6);
+    const unsigned rows = std::min<unsigned>((nc + RT * FR - 1) / (RT * FR), 148 * FB);
     const dim3 halves((nv + 255) / 256, 2);
     const bf16* t = theta_bf.p;
     feat_var_kernel<<<grid_for(nv), 256, 0, st>>>(g, B, syn, post, w.z, w.ty);
@@ -1472,18 +1567,21 @@ struct rbp_net {
     const NetWork& w = ws;
     const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
     const dim3 quarters((nv + 255) / 256, 4);
-    const int tiles = (int)std::min<unsigned>((nc + RT - 1) / RT, GRAD_BLOCKS);  // four resident blocks per SM
+    const auto tiles = [&](int stage) {
+      const unsigned n = RT * back_rows(stage);
+      return (int)std::min<unsigned>((nc + n - 1) / n, 148 * back_blocks(stage));
+    };  // four resident blocks per SM
     const int gather = (int)std::min<unsigned>((nc + 127) / 128, GRAD_BLOCKS);
     float* pg = partial;
     const bf16* t = theta_bf.p;
-    rows_backward_kernel<2><<<tiles, RT, rows_backward_smem(2), st>>>(g, nc, w, t, dr, pg);
+    rows_backward_kernel<2><<<tiles(2), RT, rows_backward_smem(2), st>>>(g, nc, w, t, dr, pg);
     dn_kernel<<<quarters, 256, 0, st>>>(g, nc, nv, t + P_G2, w.ty, w.da, w.dn);
     dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G2, w.ty, w.m2, w.n2, w.da, w.dn, w.dm2, pg + P_G2);
-    rows_backward_kernel<1><<<tiles, RT, rows_backward_smem(1), st>>>(g, nc, w, t, dr, pg);
+    rows_backward_kernel<1><<<tiles(1), RT, rows_backward_smem(1), st>>>(g, nc, w, t, dr, pg);
     dn_kernel<<<quarters, 256, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.da, w.dn);
     dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.m1, w.n1, w.da, w.dn, w.dm1, pg + P_G1);
-    rows_backward_kernel<0><<<tiles, RT, rows_backward_smem(0), st>>>(g, nc, w, t, dr, pg);
-    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 256, 0, st>>>(pg, tiles, gather, vars, grad.p, loss.p);
+    rows_backward_kernel<0><<<tiles(0), RT, rows_backward_smem(0), st>>>(g, nc, w, t, dr, pg);
+    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 256, 0, st>>>(pg, tiles(1), tiles(2), gather, vars, grad.p, loss.p);
   }
 };
 
