@@ -171,13 +171,14 @@ __global__ void feat_var_kernel(NetGraph g, long long B, const uint8_t* syn, con
 constexpr int GRAD_BLOCKS = 148 * 4;               // at most so many blocks add to a parameter
 constexpr int GRAD_STRIDE = (N_PARAMS + 1 + 3) / 4 * 4;  // the loss comes after the parameters
 constexpr int RT = 128;       // threads (rows) of a row kernel's tile
-// Rows per thread and resident blocks per SM of the row kernels: each weight read from shared
-// memory serves that many rows.  us per launch at 958,464 rows, one row at 6 (forward) and 4
-// blocks / two rows at 4 and 2: forward 108, 204, 217 / 86, 179, 192 (four rows: 108, 253, 266);
-// backward stages 0, 1, 2: 305, 250, 190 / 274, 241, 234.
-constexpr int FR = 2, FB = 4;
-__host__ __device__ constexpr int back_rows(int stage) { return stage == 2 ? 1 : 2; }
-__host__ __device__ constexpr int back_blocks(int stage) { return stage == 2 ? 4 : 2; }
+// Rows per thread of the row kernels: each weight read from shared memory serves that many rows.
+// us per launch at 958,464 rows, one row / two rows: forward stages 1-3 108, 204, 217 / 86, 178,
+// 191 (four rows: 108, 253, 266); backward stages 0-2 305, 250, 190 / 274, 240, 234.  So two,
+// one in the last of these, and one where two would leave SMs without a block: a step of 16
+// shots (14,976 rows) takes 141 us with one row and 156 with two, of 64 shots 246 and 237.
+constexpr unsigned TWO_ROWS_FROM = 148 * 2 * RT;
+__host__ __device__ constexpr int forward_blocks(int rows) { return rows == 1 ? 6 : 4; }  // resident per SM
+__host__ __device__ constexpr int backward_blocks(int rows) { return rows == 1 ? 4 : 2; }
 constexpr int SY = NH + 4;    // padded shared-memory rows of the gradient tiles
 constexpr int SX = ND + 4;
 
@@ -290,10 +291,10 @@ __device__ __forceinline__ void stage(const bf16* w, int n, float* s) {
 }
 
 // Forward of a row up to its next message (STAGE 1: x^ -> m1; 2: a1 -> m2) or readout (3: a2 -> o).
-template <int STAGE>
-__global__ void __launch_bounds__(RT, FB) rows_forward_kernel(NetGraph g, unsigned nc, unsigned nv, NetWork w,
-                                                              const bf16* theta, const uint8_t* syn,
-                                                              const float* lmean) {
+template <int STAGE, int FR>
+__global__ void __launch_bounds__(RT, forward_blocks(FR)) rows_forward_kernel(NetGraph g, unsigned nc, unsigned nv,
+                                                                              NetWork w, const bf16* theta,
+                                                                              const uint8_t* syn, const float* lmean) {
   __shared__ __align__(16) float sE[NH * 8], sW[NH * ND], sU1[NH * ND], sU2[STAGE == 3 ? NH * ND : 4];
   __shared__ float sb1[NH], sb2[NH], sO[NH];
   __shared__ __align__(16) float sG[NTY * SX];
@@ -552,10 +553,11 @@ __device__ __forceinline__ void outer_sum(const float* sy, const float* sx, int 
 //   2: dO += dout g2, dU2 += dq2 a2^T, db2 += dq2, da = U2^T dq2
 //   1: dW2 += dm2 g1^T, dU1 += dq1 a1^T, db1 += dq1, da = U1^T dq1
 //   0: dW1 += dm1 g0^T, dE += dq0 x^T
-template <int STAGE>
-__global__ void __launch_bounds__(RT, back_blocks(STAGE)) rows_backward_kernel(NetGraph g, unsigned nc, NetWork w, const bf16* theta,
-                                                               const float* dr, float* grad) {
-  constexpr int BR = back_rows(STAGE), WR = 32 * BR;  // rows of a thread, of a warp's tile
+template <int STAGE, int BR>
+__global__ void __launch_bounds__(RT, backward_blocks(BR)) rows_backward_kernel(NetGraph g, unsigned nc, NetWork w,
+                                                                                const bf16* theta, const float* dr,
+                                                                                float* grad) {
+  constexpr int WR = 32 * BR;  // rows of a warp's tile
   extern __shared__ __align__(16) float sm[];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, jq = lane >> 2, kq = lane & 3;
   float* sy = sm + warp * (WR * (SY + SX));      // this warp's [WR][SY]
@@ -757,8 +759,8 @@ __global__ void __launch_bounds__(RT, back_blocks(STAGE)) rows_backward_kernel(N
     }
   }
 }
-constexpr int rows_backward_smem(int stage) {
-  return (RT * back_rows(stage) * (SY + SX) + NH + (stage == 2 ? 1 : 2) * NH * ND + (stage == 0 ? NH * 8 : 0)) * 4;
+constexpr int rows_backward_smem(int stage, int rows) {
+  return (RT * rows * (SY + SX) + NH + (stage == 2 ? 1 : 2) * NH * ND + (stage == 0 ? NH * 8 : 0)) * 4;
 }
 
 // ------------------------------------------------------------------ readout and loss (training path)
@@ -1544,21 +1546,24 @@ struct rbp_net {
     return RBP_OK;
   }
 
+  static int rows_per_thread(unsigned nc) { return nc >= TWO_ROWS_FROM ? 2 : 1; }
+
   // Training-path forward; leaves what the backward pass needs in the workspace.
   void forward(long long B, const uint8_t* syn, const float* post, cudaStream_t st) {
     const NetGraph g = graph();
     const NetWork& w = ws;
     const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
     // weights are staged once per block: the resident blocks loop over their rows
-    const unsigned rows = std::min<unsigned>((nc + RT * FR - 1) / (RT * FR), 148 * FB);
+    const int R = rows_per_thread(nc);
+    const unsigned rows = std::min<unsigned>((nc + RT * R - 1) / (RT * R), 148 * forward_blocks(R));
     const dim3 halves((nv + 255) / 256, 2);
     const bf16* t = theta_bf.p;
     feat_var_kernel<<<grid_for(nv), 256, 0, st>>>(g, B, syn, post, w.z, w.ty);
-    rows_forward_kernel<1><<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
+    (R == 2 ? rows_forward_kernel<1, 2> : rows_forward_kernel<1, 1>)<<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
     varsum_kernel<<<halves, 256, 0, st>>>(g, nc, nv, w.m1, w.n1);
-    rows_forward_kernel<2><<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
+    (R == 2 ? rows_forward_kernel<2, 2> : rows_forward_kernel<2, 1>)<<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
     varsum_kernel<<<halves, 256, 0, st>>>(g, nc, nv, w.m2, w.n2);
-    rows_forward_kernel<3><<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
+    (R == 2 ? rows_forward_kernel<3, 2> : rows_forward_kernel<3, 1>)<<<rows, RT, 0, st>>>(g, nc, nv, w, t, syn, chk_lmean.p);
   }
 
   // Gradients of everything behind the readout (dr), summed with the readout's own into grad and loss.
@@ -1567,21 +1572,21 @@ struct rbp_net {
     const NetWork& w = ws;
     const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
     const dim3 quarters((nv + 255) / 256, 4);
-    const auto tiles = [&](int stage) {
-      const unsigned n = RT * back_rows(stage);
-      return (int)std::min<unsigned>((nc + n - 1) / n, 148 * back_blocks(stage));
-    };  // four resident blocks per SM
+    const auto blocks = [&](int rows) { return (int)std::min<unsigned>((nc + RT * rows - 1) / (RT * rows), 148 * backward_blocks(rows)); };
+    const int R = rows_per_thread(nc), tiles = blocks(R), last = blocks(1);
     const int gather = (int)std::min<unsigned>((nc + 127) / 128, GRAD_BLOCKS);
     float* pg = partial;
     const bf16* t = theta_bf.p;
-    rows_backward_kernel<2><<<tiles(2), RT, rows_backward_smem(2), st>>>(g, nc, w, t, dr, pg);
+    rows_backward_kernel<2, 1><<<last, RT, rows_backward_smem(2, 1), st>>>(g, nc, w, t, dr, pg);
     dn_kernel<<<quarters, 256, 0, st>>>(g, nc, nv, t + P_G2, w.ty, w.da, w.dn);
     dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G2, w.ty, w.m2, w.n2, w.da, w.dn, w.dm2, pg + P_G2);
-    rows_backward_kernel<1><<<tiles(1), RT, rows_backward_smem(1), st>>>(g, nc, w, t, dr, pg);
+    (R == 2 ? rows_backward_kernel<1, 2> : rows_backward_kernel<1, 1>)<<<tiles, RT, rows_backward_smem(1, R), st>>>(
+        g, nc, w, t, dr, pg);
     dn_kernel<<<quarters, 256, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.da, w.dn);
     dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.m1, w.n1, w.da, w.dn, w.dm1, pg + P_G1);
-    rows_backward_kernel<0><<<tiles(0), RT, rows_backward_smem(0), st>>>(g, nc, w, t, dr, pg);
-    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 256, 0, st>>>(pg, tiles(1), tiles(2), gather, vars, grad.p, loss.p);
+    (R == 2 ? rows_backward_kernel<0, 2> : rows_backward_kernel<0, 1>)<<<tiles, RT, rows_backward_smem(0, R), st>>>(
+        g, nc, w, t, dr, pg);
+    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 256, 0, st>>>(pg, tiles, last, gather, vars, grad.p, loss.p);
   }
 };
 
@@ -1638,10 +1643,12 @@ int rbp_net_create(const rbp_graph* g, const float* llr, rbp_net** out) {
     return rc;
   }
   to_bf16_kernel<<<4, 256>>>(N_PARAMS, n->theta.p, n->theta_bf.p);
-  for (const void* k : {reinterpret_cast<const void*>(rows_backward_kernel<0>),
-                        reinterpret_cast<const void*>(rows_backward_kernel<1>),
-                        reinterpret_cast<const void*>(rows_backward_kernel<2>)})
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_backward_smem(0)) != cudaSuccess) {
+  for (const void* k : {reinterpret_cast<const void*>(rows_backward_kernel<0, 1>),
+                        reinterpret_cast<const void*>(rows_backward_kernel<0, 2>),
+                        reinterpret_cast<const void*>(rows_backward_kernel<1, 1>),
+                        reinterpret_cast<const void*>(rows_backward_kernel<1, 2>),
+                        reinterpret_cast<const void*>(rows_backward_kernel<2, 1>)})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_backward_smem(0, 2)) != cudaSuccess) {
       delete n;
       return fail(RBP_ERR_CUDA, "rbp_net_create: cannot reserve shared memory for the training kernels");
     }

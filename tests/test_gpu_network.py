@@ -65,6 +65,16 @@ def test_inference_matches_specification(size):
 @pytest.mark.parametrize("B", [1, 37])
 @pytest.mark.parametrize("size", SIZES)
 def test_gradients_match_specification(size, B):
+    _check_gradients(size, B)
+
+
+# 37,888 rows (checks times shots) is where a thread takes two: below, at, and past it with a ragged end
+@pytest.mark.parametrize("size,B", [((37, 64, 8, 3), 1023), ((37, 64, 8, 3), 1024), ((131, 300, 8, 3), 301)])
+def test_gradients_match_specification_rows_per_thread(size, B):
+    _check_gradients(size, B)
+
+
+def _check_gradients(size, B):
     H, dec, net, theta, syn, post = _setup(size, B)
     target = np.random.default_rng(3).integers(0, 2, (B, H.shape[1])).astype(np.uint8)
     loss = torch.zeros(1, device=DEV)
