@@ -163,7 +163,7 @@ __global__ void feat_var_kernel(NetGraph g, long long B, const uint8_t* syn, con
 // Arrays are stored in 16-byte columns ([chunk][row]), so a warp's accesses are
 // contiguous.  With one thread per output element, each layer re-reading and re-writing
 // the node states (245 MB each for 1,024 shots of the 936 x 2,592 graph), a step of
-// 1,024 shots took 9.71 ms; now 1.82.
+// 1,024 shots took 9.71 ms; now 1.78.
 
 // Gradients are summed in three steps: fp32 within a block (over its rows), one partial sum
 // per block in memory, and the blocks' sums in double.  With an atomic add per block the
@@ -809,22 +809,23 @@ __global__ void __launch_bounds__(256) readout_kernel(NetGraph g, long long B, c
   }
 }
 
-// The blocks' partial sums of each parameter (and of the loss), added in double: 8 warps share
-// 32 parameters.  rows / last / gates / vars: blocks of the kernels behind a parameter (last: the
+// The blocks' partial sums of each parameter (and of the loss), added in double: 32 warps share
+// 32 parameters, so that the latency of a few loads bounds the kernel (8 warps: 36 us for 592
+// rows of partial sums, now 11).  rows / last / gates / vars: blocks of the kernels behind a parameter (last: the
 // second layer's update and readout).
-__global__ void __launch_bounds__(256) grad_sum_kernel(const float* partial, int rows, int last, int gates, int vars,
+__global__ void __launch_bounds__(1024) grad_sum_kernel(const float* partial, int rows, int last, int gates, int vars,
                                                        float* grad, float* loss) {
-  __shared__ double part[8][32];
+  __shared__ double part[32][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
   const bool gate = (p >= P_G1 && p < P_U1) || (p >= P_G2 && p < P_U2);
   const int n = p > N_PARAMS ? 0 : (gate ? gates : (p >= P_OZ ? vars : (p >= P_U2 ? last : rows)));
   double s = 0.0;
 #pragma unroll 4
-  for (int k = warp; k < n; k += 8) s += (double)partial[(size_t)k * GRAD_STRIDE + p];
+  for (int k = warp; k < n; k += 32) s += (double)partial[(size_t)k * GRAD_STRIDE + p];
   part[warp][lane] = s;
   __syncthreads();
   if (warp == 0 && p <= N_PARAMS) {
-    for (int k = 1; k < 8; ++k) s += part[k][lane];
+    for (int k = 1; k < 32; ++k) s += part[k][lane];
     if (p < N_PARAMS) grad[p] = (float)s;
     else *loss = (float)s;
   }
@@ -1586,7 +1587,7 @@ struct rbp_net {
     dm_kernel<<<gather, 512, 0, st>>>(g, nc, nv, t + P_G1, w.ty, w.m1, w.n1, w.da, w.dn, w.dm1, pg + P_G1);
     (R == 2 ? rows_backward_kernel<0, 2> : rows_backward_kernel<0, 1>)<<<tiles, RT, rows_backward_smem(0, R), st>>>(
         g, nc, w, t, dr, pg);
-    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 256, 0, st>>>(pg, tiles, last, gather, vars, grad.p, loss.p);
+    grad_sum_kernel<<<(N_PARAMS + 32) / 32, 1024, 0, st>>>(pg, tiles, last, gather, vars, grad.p, loss.p);
   }
 };
 
