@@ -66,9 +66,9 @@ LEARNED_LEGS = 4
 # DRAM bytes (read + write) of the two decode-kernel launches of one learned decode, per shot: ncu
 # dram__bytes_read.sum + dram__bytes_write.sum on 16,384 shots of this workload with the committed
 # kernel shape (python -m pelagos_b200.experiments decode-case --shots 16384 --learned
-# --launch 448,1,1,2), 378,680,320 B / 16,384.  At this size L2 keeps part of the saved states
+# --launch 448,1,1,2), 380,889,536 B / 16,384.  At this size L2 keeps part of the saved states
 # between the two launches; the states and I/O a shot must move at any size come to about 26.6 KB.
-DECODE_DRAM_BYTES_PER_SHOT = 23113
+DECODE_DRAM_BYTES_PER_SHOT = 23247
 
 
 def algorithmic_bytes_per_shot_iteration(C: int, V: int, E: int, msg_bytes: int = 4) -> int:
@@ -486,7 +486,7 @@ def main():
                     "per_call": {"value": whole_job_shots_per_s(world, shots, call_ms),
                                  "api": "LearnedRelayBPDecoder.decode per batch, results copied to pinned "
                                         "host memory before the next call", "steps": call_steps}},
-            "gpu_launches": args.steps * 3,
+            "gpu_launches": args.steps * 5,  # pre-iterations, queue order, network, relay legs, result arrays
             "roofline": {"bound": "smem", "achieved": achieved, "peak": smem_peak, "unit": "GB/s",
                          "frac": achieved / smem_peak, "traffic": dram_bytes,
                          "kernel": "relaybp decode kernel (pre-iterations + relay legs of one learned step)",

@@ -107,11 +107,12 @@ RBP_API int rbp_decoder_set_llr(rbp_decoder* d, const float* llr);
 /* Launch shape (no reference counterpart: the reference autotunes Triton
  * tile sizes instead, src/pelagos/autotune.py:302-541).  A group of
  * `group_threads` threads (a multiple of 32, at most 1024) decodes
- * `shots_per_group` shots at once (1 or 2) and a thread block holds
- * `groups_per_block` such groups.  groups_per_block 1, or two shots per
- * group, selects the block-per-group kernel (check degrees up to 16); 0 (or
- * -1) the kernel whose blocks hold as many one-shot groups as fit.  Zeros pick
- * the defaults.  Results do not depend on the shape.  Fails with
+ * one shot at a time and a thread block holds `groups_per_block` such groups;
+ * 0 (or -1): as many as fit.  shots_per_group (1 or 2) is kept for callers
+ * that set it: 2 asks for one group per block with room for two shots, under
+ * the register and memory limits of two, and decodes them one after another.
+ * All zeros: the library chooses by the code's size and each batch's size.
+ * Results do not depend on the shape.  Fails with
  * RBP_ERR_UNSUPPORTED when the shape's registers or shared memory do not fit.
  * Sets the shape of every launch kind (rbp_decoder_configure_kind with
  * RBP_LAUNCH_ALL and one resident block per SM). */
@@ -127,8 +128,8 @@ RBP_API int rbp_decoder_configure(rbp_decoder* d, int32_t group_threads, int32_t
 #define RBP_LAUNCH_LEGS 2
 
 /* Launch shape of one launch kind (no reference counterpart, like
- * rbp_decoder_configure).  blocks_per_sm 2 selects the block-per-group kernel
- * compiled for two resident blocks per SM (groups_per_block 1 and
+ * rbp_decoder_configure).  blocks_per_sm 2 selects the one-group-per-block
+ * kernel compiled for two resident blocks per SM (groups_per_block 1 and
  * shots_per_group 1 only; half the register file per block, so
  * group_threads is at most 512 for up to 4 owned variables per thread, 448
  * for 6, 384 for 8 and 256 for 12 or 16): two shots decode side by side on an
@@ -199,10 +200,8 @@ typedef struct {
   float solved_gamma;
   int32_t solved_legs;
   int32_t suspend_unsolved;
-  /* When to test an iteration's parity before its min-sum pass, skipping that
-   * pass when every check holds: 0 never (one fused pass), 1 at the first
-   * testable iteration of each relay leg, 2 at every iteration.  Results do
-   * not depend on it; it pays off where legs converge at once. */
+  /* 0, 1 or 2; not read.  Every iteration's convergence is tested before the
+   * next min-sum pass (what 2 asked for).  Results never depended on it. */
   int32_t parity_first;
 } rbp_batch;
 

@@ -2,11 +2,11 @@
 
 The kernel's shape is (group_threads, groups_per_block, shots_per_group[,
 blocks_per_sm]): how many threads share one shot (and so how many variables
-and checks each thread owns), how many groups a thread block holds, how many
-shots a group decodes at once (1: relaybp_decode_kernel; 2: relaybp_slots_kernel,
-one group per block), and for one-shot block-per-group launches how many
-blocks the kernel is compiled to keep resident per SM (2: half the register
-file each, two shots side by side with their own barriers).  The launches
+and checks each thread owns), how many groups a thread block holds, the shots
+per group the shape is checked for (2: one group per block under two shots'
+limits; the shots are decoded one after another), and for launches with one
+group per block how many blocks the kernel is compiled to keep resident per SM
+(2: half the register file each, two shots side by side with their own barriers).  The launches
 that run only the pre-iterations may have their own shape (``kind="pre"``).  ``tune`` times candidate shapes on a sample batch with CUDA events
 (the median of ``repeats`` timed runs after a warm-up, by default of
 ``decoder.decode`` and optionally of any decode call, e.g. a learned decode)
@@ -16,10 +16,10 @@ the reference keys its tuning cache (src/pelagos/autotune.py:130-133, 222-541):
 
 * cache file: ``$PELAGOS_B200_TUNE_CACHE`` or ``~/.cache/pelagos_b200_tune.json``;
 * candidates: every warp multiple G from 32 to 1024 that gives at most 16
-  variables and 32 checks per thread, with the multi-group kernel (the largest
-  group count that fits and, for one-warp groups, also 8) and with the
-  block-per-group kernel (one and two shots per group, and one shot per group
-  at two resident blocks per SM);
+  variables and 32 checks per thread, with several groups per block (the largest
+  group count that fits and, for one-warp groups, also 8) and with one group
+  per block (at one resident block per SM, also in the two-shot form, and at
+  two);
 * a candidate the library rejects (shared memory, registers) is skipped.
 
 ``default_shape`` returns the shape measured best for a workload and

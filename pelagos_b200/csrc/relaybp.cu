@@ -1,6 +1,6 @@
 // C ABI of the Relay-BP-S decoder (include/relaybp.h): graph preparation,
 // decoder state, launch-shape selection and the decode launch.  The kernel
-// itself is in relaybp_kernel.cuh.
+// itself is in relaybp_decode.cuh.
 
 #include "relaybp.h"
 #include "relaybp_host.h"

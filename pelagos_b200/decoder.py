@@ -175,8 +175,9 @@ class RelayBPDecoder:
     * ``mix_rounding``: rounding of the memory mix (1-g)*llr + g*posterior:
       "separate" (default; one rounding per operation), "fma_gp" or "fma_lp";
     * ``launch``: optional (group_threads, groups_per_block[, shots_per_group[, blocks_per_sm]])
-      kernel shape of every launch; shots_per_group 2 selects the kernel whose groups decode two
-      shots at once, blocks_per_sm 2 the one-shot kernel compiled for two resident blocks per SM.
+      kernel shape of every launch (by default the library chooses by the code's size and each
+      batch's); blocks_per_sm 2 selects the kernel compiled for two resident blocks per SM, and
+      shots_per_group 2 (one group per block, under two shots' limits) changes nothing else.
       ``configure_launch(..., kind="pre")`` gives the pre-iteration launches their own shape.
     * ``hard_shots_first`` (default True): a relay decode of at least 1024 shots
       runs as two launches, the pre-iterations and then the relay legs resumed
@@ -184,12 +185,8 @@ class RelayBPDecoder:
       unconverged queued first.  Those few shots run up to
       pre_iter + num_sets * set_max_iter iterations; started first, they finish
       alongside the bulk instead of after it.  Results are identical.
-    * ``parity_first`` (default 2): when the kernel tests an iteration's parity
-      on its own before the min-sum pass, skipping that pass once every check
-      holds — 0 never (one fused pass), 1 at the first testable iteration of
-      each relay leg, 2 at every iteration.  Results are identical; 2 measured
-      fastest (27.4 vs 28.2 ms plain, 20.0 vs 21.3 ms learned, 65,536 shots of
-      the [[144,12,12]] phenomenological code).
+    * ``parity_first`` (0, 1 or 2): accepted and without effect; the kernel tests
+      every iteration's convergence before the next min-sum pass.
     * ``cuda_graph`` (default False): a one-GPU decode of at least 1024 shots
       with no per-call options replays a CUDA graph of its launches, captured
       on the first call of each batch size (and again after a launch-shape
