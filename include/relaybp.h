@@ -398,6 +398,18 @@ RBP_API int rbp_gf2_matvec(const uint8_t* x, int64_t B, int32_t N, const int32_t
                            int32_t R, uint8_t* out, void* stream);
 
 /*
+ * Failure counts of B decoded shots: counts[4] = shots whose estimate flips an
+ * observable (a row of the [R, N] matrix with odd parity over errors XOR
+ * estimates) or that have no solution (found_count <= 0), shots without one,
+ * shots with one that flip, and the sum of iterations.  Device pointers, rows
+ * of N bytes (the low bit counts); asynchronous on `stream`.  Sizes must be
+ * positive, N at most 49,152.
+ */
+RBP_API int rbp_gf2_failures(const uint8_t* errors, const uint8_t* estimates, int64_t B, int32_t N,
+                             const int32_t* row_ptr, const int32_t* cols, int32_t R, const int32_t* found_count,
+                             const int32_t* iterations, int64_t* counts, void* stream);
+
+/*
  * Result arrays of a decode in one launch (asynchronous on `stream`, device
  * pointers; src/pelagos/decoder.py:3839-3873): weights [B] (float, or double
  * with weights_f64 = 1; weight_fixed * 2^-32, +inf where it is INT64_MAX),

@@ -65,6 +65,7 @@ EXPORTED_SYMBOLS = (
     "rbp_net_train_step",
     "rbp_net_propose",
     "rbp_gf2_matvec",
+    "rbp_gf2_failures",
     "rbp_results",
     "rbp_queue_order",
 )
@@ -223,6 +224,8 @@ def _declare(lib):
     lib.rbp_net_propose.argtypes = [P, i64, P, P, i64, ct.c_float, ct.c_float, P, P, P, P, P]
     lib.rbp_gf2_matvec.restype = ct.c_int
     lib.rbp_gf2_matvec.argtypes = [P, i64, i32, P, P, i32, P, P]
+    lib.rbp_gf2_failures.restype = ct.c_int
+    lib.rbp_gf2_failures.argtypes = [P, P, i64, i32, P, P, i32, P, P, P, P]
     lib.rbp_results.restype = ct.c_int
     lib.rbp_results.argtypes = [P, P, i64, i32, P, i32, P, P, P, P]
     lib.rbp_queue_order.restype = ct.c_int

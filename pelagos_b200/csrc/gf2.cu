@@ -134,7 +134,102 @@ int launch_rows(const uint8_t* x, long long B, int N, const int* row_ptr, const 
   return RBP_OK;
 }
 
+// Failure counts of decoded shots: a shot flips when some row of the observables has odd parity over
+// e XOR est, so both arrays are read once, XORed as column words, and nothing but four sums leaves
+// the kernel.  counts += (flipped or unsolved, unsolved, flipped but solved, iterations); integer
+// adds, so the order of the blocks does not matter.  Bound by reading the two arrays: 65,536
+// shots of 2,592 columns, 12 observables 79 us (340 MB at 4.3 TB/s), against 190 us for two
+// products of 42 us and a dozen elementwise launches and sums over their results.
+template <int IN, bool WARP_ROWS>
+__global__ void __launch_bounds__(GF2_THREADS) gf2_failures_kernel(const uint8_t* e, const uint8_t* est, long long B,
+                                                                 int tile, int N, const int* row_ptr, const int* cols,
+                                                                 int R, const int* found, const int* iters,
+                                                                 unsigned long long* counts) {
+  extern __shared__ uint32_t word[];  // [N rounded up to 32]
+  __shared__ uint32_t s_flip;         // bit b: some observable of the tile's shot b flips
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = GF2_THREADS / 32;
+  long long n_fail = 0, n_unsolved = 0, n_flip = 0, n_iter = 0;  // warp 0: its lane's shots
+  for (long long b0 = blockIdx.x * (long long)tile; b0 < B; b0 += gridDim.x * (long long)tile) {
+    const int nb = (int)min((long long)tile, B - b0);
+    const long long at = (b0 + min(lane, nb - 1)) * N;
+    for (int j0 = warp * 32; j0 < N; j0 += nwarps * 32) {
+      const uint32_t w = lane < nb ? load_columns<IN>(e + at, j0, N) ^ load_columns<IN>(est + at, j0, N) : 0u;
+      word[j0 + lane] = transpose32(w, lane);
+    }
+    if (threadIdx.x == 0) s_flip = 0u;
+    __syncthreads();
+    uint32_t any = 0u;
+    if constexpr (WARP_ROWS) {
+      for (int r = warp; r < R; r += nwarps) {
+        uint32_t p = 0u;
+        for (int k = row_ptr[r] + lane; k < row_ptr[r + 1]; k += 32) p ^= word[cols[k]];
+        any |= __reduce_xor_sync(0xffffffffu, p);
+      }
+    } else {
+      for (int r = threadIdx.x; r < R; r += GF2_THREADS) {
+        uint32_t p = 0u;
+        for (int k = row_ptr[r]; k < row_ptr[r + 1]; ++k) p ^= word[cols[k]];
+        any |= p;
+      }
+      any = __reduce_or_sync(0xffffffffu, any);
+    }
+    if (lane == 0 && any) atomicOr(&s_flip, any);
+    __syncthreads();  // also: the next tile overwrites the words
+    if (warp == 0) {
+      if (lane < nb) {
+        const bool flip = (s_flip >> lane) & 1u, unsolved = __ldg(found + b0 + lane) <= 0;
+        n_fail += flip || unsolved;
+        n_unsolved += unsolved;
+        n_flip += flip && !unsolved;
+        n_iter += __ldg(iters + b0 + lane);
+      }
+      __syncwarp();  // s_flip is read before the next tile clears it
+    }
+  }
+  if (warp == 0) {
+    long long n[4] = {n_fail, n_unsolved, n_flip, n_iter};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) n[i] += __shfl_xor_sync(0xffffffffu, n[i], o);
+      if (lane == 0 && n[i]) atomicAdd(counts + i, (unsigned long long)n[i]);
+    }
+  }
+}
+
+template <int IN>
+int launch_failures(const uint8_t* e, const uint8_t* est, long long B, int N, const int* row_ptr, const int* cols, int R,
+                    const int* found, const int* iters, unsigned long long* counts, cudaStream_t st) {
+  const size_t smem = (size_t)((N + 31) / 32 * 32) * sizeof(uint32_t);
+  auto kernel = R < 64 ? gf2_failures_kernel<IN, true> : gf2_failures_kernel<IN, false>;  // as launch_rows
+  if (smem > 48 * 1024 - 64)
+    RBP_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem));
+  const long long spread = 148LL * 4;
+  const int tile = (int)std::min<long long>(GF2_SHOTS, std::max<long long>(1, (B + spread - 1) / spread));
+  const int blocks = (int)std::min<long long>((B + tile - 1) / tile, 148LL * 8);
+  RBP_CUDA(cudaMemsetAsync(counts, 0, 4 * sizeof(unsigned long long), st));
+  kernel<<<blocks, GF2_THREADS, smem, st>>>(e, est, B, tile, N, row_ptr, cols, R, found, iters, counts);
+  RBP_CUDA(cudaGetLastError());
+  return RBP_OK;
+}
+
 }  // namespace
+
+extern "C" int rbp_gf2_failures(const uint8_t* errors, const uint8_t* estimates, int64_t B, int32_t N,
+                                const int32_t* row_ptr, const int32_t* cols, int32_t R, const int32_t* found_count,
+                                const int32_t* iterations, int64_t* counts, void* stream) {
+  if (B <= 0 || N <= 0 || R <= 0) return fail(RBP_ERR_ARGUMENT, "rbp_gf2_failures: sizes must be positive");
+  if (!errors || !estimates || !row_ptr || !cols || !found_count || !iterations || !counts)
+    return fail(RBP_ERR_ARGUMENT, "rbp_gf2_failures: null buffer");
+  if (N > 48 * 1024) return fail(RBP_ERR_UNSUPPORTED, "rbp_gf2_failures: rows longer than 49,152 columns");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const uintptr_t in = reinterpret_cast<uintptr_t>(errors) | reinterpret_cast<uintptr_t>(estimates) | (uintptr_t)N;
+  unsigned long long* n = reinterpret_cast<unsigned long long*>(counts);
+  if (in % 16 == 0) return launch_failures<16>(errors, estimates, B, N, row_ptr, cols, R, found_count, iterations, n, st);
+  if (in % 4 == 0) return launch_failures<4>(errors, estimates, B, N, row_ptr, cols, R, found_count, iterations, n, st);
+  return launch_failures<1>(errors, estimates, B, N, row_ptr, cols, R, found_count, iterations, n, st);
+}
 
 extern "C" int rbp_gf2_matvec(const uint8_t* x, int64_t B, int32_t N, const int32_t* row_ptr, const int32_t* cols,
                               int32_t R, uint8_t* out, void* stream) {

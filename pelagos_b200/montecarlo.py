@@ -86,6 +86,15 @@ class MonteCarlo:
 
     def failures(self, e: torch.Tensor, out: dict):
         """Device counts (failures, unconverged, logical flips) of one decoded batch."""
+        est, found, iters = out["errors"], out["found_count"], out["iterations"]
+        B = e.shape[0]
+        # a decoder's own outputs take one launch; anything else (other types, layouts, empty) the general products
+        if (B and self.O.R and self.O.cols.numel() and e.shape == est.shape == (B, self.V)
+                and found.shape == iters.shape == (B,)
+                and e.dtype == est.dtype == torch.uint8 and found.dtype == iters.dtype == torch.int32
+                and all(x.is_contiguous() and x.device == e.device for x in (e, est, found, iters))
+                and e.device == self.O.cols.device):
+            return self.O.failures(e, est, found, iters)
         flip = (self.O.apply(e) != self.O.apply(out["errors"].to(torch.uint8))).any(dim=1)
         unconv = out["found_count"] <= 0
         return torch.stack([(flip | unconv).sum(), unconv.sum(), (flip & ~unconv).sum(),

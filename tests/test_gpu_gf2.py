@@ -9,6 +9,7 @@ import scipy.sparse as sp
 import torch
 
 from pelagos_b200.adapter import _DeviceCSR
+from pelagos_b200.montecarlo import MonteCarlo
 
 pytestmark = pytest.mark.gpu
 
@@ -25,3 +26,32 @@ def test_matches_integer_product(B, N, R, offset):
     got = _DeviceCSR(A, x.device).apply(x).cpu().numpy()
     want = (A.astype(np.int64) @ (x.cpu().numpy().T.astype(np.int64) & 1)).T % 2
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("offset", [0, 4, 1])
+@pytest.mark.parametrize("B,N,R", [(1, 33, 5), (31, 64, 64), (33, 100, 70), (1185, 2592, 12), (20000, 48, 63),
+                                   (40, 49152, 3), (70, 16, 300), (5, 1, 1)])
+def test_failure_counts_match_the_general_products(B, N, R, offset):
+    rng = np.random.default_rng(B + N)
+    O = sp.random(R, N, density=min(1.0, 3 / N), format="csr", random_state=2, dtype=np.float64)
+    O.data[:] = 1
+    O[0, N - 1] = 1
+    mc = MonteCarlo(sp.csr_matrix(np.ones((1, N))), np.full(N, 0.1), O)
+    buf = torch.from_numpy(rng.integers(0, 256, size=2 * B * N + 32, dtype=np.uint8)).cuda()  # only low bits count
+    e = buf[offset:offset + B * N].view(B, N)
+    est = buf[B * N + 16 + offset:2 * B * N + 16 + offset].view(B, N)
+    est[: B // 2] = e[: B // 2]  # half of the shots do not flip
+    if B > 2:
+        est[1, N - 1] ^= 1  # one whose only difference is the last column
+    found = torch.from_numpy(rng.integers(0, 3, size=B).astype(np.int32)).cuda()
+    iters = torch.from_numpy(rng.integers(0, 6081, size=B).astype(np.int32)).cuda()
+    got = mc.failures(e, {"errors": est, "found_count": found, "iterations": iters}).cpu().numpy()
+    A = O.astype(np.int64)
+    d = (e.cpu().numpy() ^ est.cpu().numpy()).astype(np.int64) & 1
+    flip = ((A @ d.T) % 2).any(axis=0)
+    unsolved = found.cpu().numpy() <= 0
+    want = [(flip | unsolved).sum(), unsolved.sum(), (flip & ~unsolved).sum(), iters.cpu().numpy().astype(np.int64).sum()]
+    np.testing.assert_array_equal(got, want)
+    # int64 counts take the general products
+    other = mc.failures(e, {"errors": est, "found_count": found.long(), "iterations": iters.long()})
+    np.testing.assert_array_equal(other.cpu().numpy(), want)
