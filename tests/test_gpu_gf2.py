@@ -28,6 +28,13 @@ def test_matches_integer_product(B, N, R, offset):
     np.testing.assert_array_equal(got, want)
 
 
+# rows staged as whole 16-byte pieces: the shortest and longest, a half word at the end, one shot, and past the limit
+@pytest.mark.parametrize("B,N,R", [(1, 32, 5), (33, 48, 70), (1300, 2608, 12), (40, 12288, 70), (40, 12304, 70)])
+def test_staged_rows_match_integer_product(B, N, R):
+    test_matches_integer_product(B, N, R, 0)
+    test_failure_counts_match_the_general_products(B, N, R, 0)
+
+
 @pytest.mark.parametrize("offset", [0, 4, 1])
 @pytest.mark.parametrize("B,N,R", [(1, 33, 5), (31, 64, 64), (33, 100, 70), (1185, 2592, 12), (20000, 48, 63),
                                    (40, 49152, 3), (70, 16, 300), (5, 1, 1)])
