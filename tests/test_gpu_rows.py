@@ -93,3 +93,19 @@ def test_special_priors_match_oracle(dtype):
         out = dec.decode(torch.from_numpy(syn).to(DEV), prior_llr=torch.from_numpy(pl).to(DEV),
                          return_last_posterior=True)
         _compare(dec, out, _oracle(dec, syn, "separate", llr_per_shot=pl))
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16", "float64"])
+@pytest.mark.parametrize("size", [(40, 90, 8, 3), (33, 70, 16, 8), (24, 60, 20, 5)])
+def test_legs_with_per_shot_priors_match_oracle(size, dtype):
+    """Many short legs: the first pass from the shot's messages, later ones from its kept sums, converging or not."""
+    H = _graph(*size, seed=size[0])
+    syn = _syndromes(H, 0.04, 40, seed=6)
+    syn[:4] = np.random.default_rng(8).integers(0, 2, (4, size[0]))  # shots whose legs do not converge
+    pl = (3.0 + np.random.default_rng(9).normal(0, 1, (40, size[1]))).astype(np.float32)
+    for shape in SHAPES if size[2] <= 16 else SHAPES[:2]:
+        dec = RelayBPDecoder(H, np.full(size[1], 0.03), data_type=dtype, launch=shape,
+                             **{**BASE, "num_sets": 9, "set_max_iter": 4, "stop_nconv": 6})
+        out = dec.decode(torch.from_numpy(syn).to(DEV), prior_llr=torch.from_numpy(pl).to(DEV),
+                         return_last_posterior=True)
+        _compare(dec, out, _oracle(dec, syn, "separate", llr_per_shot=pl))
