@@ -393,6 +393,9 @@ RBP_API int rbp_net_propose(rbp_net* n, int64_t B, const uint8_t* syn, const flo
  * XOR_{j in row r} x[b, j] (device uint8 [B, R]).  Replaces the host-side
  * products of the reference's observable runner, s = H e and O e
  * (src/pelagos/adapter.py:545-560, 601-613, 679).  N <= 49,152.
+ *
+ * This and the three entries below take no handle: they launch on the calling
+ * thread's current device, which has to be the buffers' (and the stream's).
  */
 RBP_API int rbp_gf2_matvec(const uint8_t* x, int64_t B, int32_t N, const int32_t* row_ptr, const int32_t* cols,
                            int32_t R, uint8_t* out, void* stream);

@@ -77,18 +77,20 @@ class _DeviceCSR:
         x = x.to(dtype=torch.uint8).contiguous()
         B = int(x.shape[0])
         out = torch.empty(B, self.R, dtype=torch.uint8, device=x.device)
-        nat.check(nat.lib().rbp_gf2_matvec(_ptr(x), B, self.N, _ptr(self.row_ptr), _ptr(self.cols), self.R,
-                                           _ptr(out), ct.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)),
-                  "rbp_gf2_matvec")
+        with torch.cuda.device(x.device):  # the entry launches on the current device
+            nat.check(nat.lib().rbp_gf2_matvec(_ptr(x), B, self.N, _ptr(self.row_ptr), _ptr(self.cols), self.R,
+                                               _ptr(out), ct.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)),
+                      "rbp_gf2_matvec")
         return out
 
     def failures(self, e: torch.Tensor, est: torch.Tensor, found: torch.Tensor, iters: torch.Tensor) -> torch.Tensor:
         """rbp_gf2_failures of [B, N] uint8 errors and estimates, int32 found counts and iterations."""
         counts = torch.empty(4, dtype=torch.int64, device=e.device)
-        nat.check(nat.lib().rbp_gf2_failures(_ptr(e), _ptr(est), int(e.shape[0]), self.N, _ptr(self.row_ptr),
-                                             _ptr(self.cols), self.R, _ptr(found), _ptr(iters), _ptr(counts),
-                                             ct.c_void_p(torch.cuda.current_stream(e.device).cuda_stream)),
-                  "rbp_gf2_failures")
+        with torch.cuda.device(e.device):
+            nat.check(nat.lib().rbp_gf2_failures(_ptr(e), _ptr(est), int(e.shape[0]), self.N, _ptr(self.row_ptr),
+                                                 _ptr(self.cols), self.R, _ptr(found), _ptr(iters), _ptr(counts),
+                                                 ct.c_void_p(torch.cuda.current_stream(e.device).cuda_stream)),
+                      "rbp_gf2_failures")
         return counts
 
 

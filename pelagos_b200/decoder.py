@@ -71,27 +71,30 @@ def _ptr(t: Optional[torch.Tensor]):
 HARD_FIRST_MIN_BATCH = 1024
 
 def finish_results(found: torch.Tensor, wfix: torch.Tensor, stop_nconv: int, weights_dtype=torch.float32):
-    """(weights, valid mask, unconverged indices) of a decode's device counts and exact weights, on the
-    current device and stream; reading the number of unconverged shots synchronises the host."""
+    """(weights, valid mask, unconverged indices) of a decode's device counts and exact weights, on their
+    device and its current stream; reading the number of unconverged shots synchronises the host."""
     B, dev = int(found.shape[0]), found.device
     weights = torch.empty(B, dtype=weights_dtype, device=dev)
     valid = torch.empty(B, dtype=torch.bool, device=dev)
     unconverged = torch.empty(B + 1, dtype=torch.int32, device=dev)  # their number comes after the capacity
     f64 = 1 if weights_dtype == torch.float64 else 0
     u = unconverged.data_ptr()
-    nat.check(nat.lib().rbp_results(found.data_ptr(), wfix.data_ptr(), B, int(stop_nconv), weights.data_ptr(), f64,
-                                    valid.data_ptr(), u, u + 4 * B, torch.cuda.current_stream(dev).cuda_stream),
-              "rbp_results")
+    with torch.cuda.device(dev):  # the entry launches on the current device
+        nat.check(nat.lib().rbp_results(found.data_ptr(), wfix.data_ptr(), B, int(stop_nconv), weights.data_ptr(), f64,
+                                        valid.data_ptr(), u, u + 4 * B, torch.cuda.current_stream(dev).cuda_stream),
+                  "rbp_results")
     return weights, valid, unconverged[:int(unconverged[B])]
 
 
 def queue_order(found: torch.Tensor, count: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Shot order with the shots that have no solution first (their number in ``count``), on the
-    current stream."""
-    order = torch.empty(found.shape[0], dtype=torch.int32, device=found.device)
-    nat.check(nat.lib().rbp_queue_order(found.data_ptr(), int(found.shape[0]), order.data_ptr(),
-                                        count.data_ptr() if count is not None else None,
-                                        torch.cuda.current_stream(found.device).cuda_stream), "rbp_queue_order")
+    device of ``found`` and its current stream."""
+    dev = found.device
+    order = torch.empty(found.shape[0], dtype=torch.int32, device=dev)
+    with torch.cuda.device(dev):  # as above
+        nat.check(nat.lib().rbp_queue_order(found.data_ptr(), int(found.shape[0]), order.data_ptr(),
+                                            count.data_ptr() if count is not None else None,
+                                            torch.cuda.current_stream(dev).cuda_stream), "rbp_queue_order")
     return order
 
 
