@@ -29,7 +29,7 @@ import scipy.sparse as sp
 import torch
 
 from . import _native as nat
-from .decoder import RelayBPDecoder, _ptr
+from .decoder import RelayBPDecoder, _ptr, on_device
 
 _DTYPE_ALIASES = {"float": "float32", "half": "float16", "double": "float64", "fp16": "float16",
                   "fp32": "float32", "fp64": "float64", "bf16": "bfloat16"}
@@ -77,7 +77,7 @@ class _DeviceCSR:
         x = x.to(dtype=torch.uint8).contiguous()
         B = int(x.shape[0])
         out = torch.empty(B, self.R, dtype=torch.uint8, device=x.device)
-        with torch.cuda.device(x.device):  # the entry launches on the current device
+        with on_device(x.device):
             nat.check(nat.lib().rbp_gf2_matvec(_ptr(x), B, self.N, _ptr(self.row_ptr), _ptr(self.cols), self.R,
                                                _ptr(out), ct.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)),
                       "rbp_gf2_matvec")
@@ -86,7 +86,7 @@ class _DeviceCSR:
     def failures(self, e: torch.Tensor, est: torch.Tensor, found: torch.Tensor, iters: torch.Tensor) -> torch.Tensor:
         """rbp_gf2_failures of [B, N] uint8 errors and estimates, int32 found counts and iterations."""
         counts = torch.empty(4, dtype=torch.int64, device=e.device)
-        with torch.cuda.device(e.device):
+        with on_device(e.device):
             nat.check(nat.lib().rbp_gf2_failures(_ptr(e), _ptr(est), int(e.shape[0]), self.N, _ptr(self.row_ptr),
                                                  _ptr(self.cols), self.R, _ptr(found), _ptr(iters), _ptr(counts),
                                                  ct.c_void_p(torch.cuda.current_stream(e.device).cuda_stream)),

@@ -26,6 +26,8 @@ from __future__ import annotations
 from typing import Dict, List, Optional, Sequence, Tuple, Union
 
 import ctypes as ct
+from contextlib import nullcontext
+
 import numpy as np
 import torch
 from scipy.sparse import csr_matrix
@@ -70,6 +72,14 @@ def _ptr(t: Optional[torch.Tensor]):
 #: Batches at least this large decode with the unconverged shots queued first (hard_shots_first).
 HARD_FIRST_MIN_BATCH = 1024
 
+def on_device(device: torch.device):
+    """Context in which ``device`` is the current one: native entries without a handle launch on the current
+    device.  Nothing to enter where it is already (0.3 us against 2 us for torch.cuda.device)."""
+    if torch.cuda.current_device() == device.index:
+        return nullcontext()
+    return torch.cuda.device(device)
+
+
 def finish_results(found: torch.Tensor, wfix: torch.Tensor, stop_nconv: int, weights_dtype=torch.float32):
     """(weights, valid mask, unconverged indices) of a decode's device counts and exact weights, on their
     device and its current stream; reading the number of unconverged shots synchronises the host."""
@@ -79,7 +89,7 @@ def finish_results(found: torch.Tensor, wfix: torch.Tensor, stop_nconv: int, wei
     unconverged = torch.empty(B + 1, dtype=torch.int32, device=dev)  # their number comes after the capacity
     f64 = 1 if weights_dtype == torch.float64 else 0
     u = unconverged.data_ptr()
-    with torch.cuda.device(dev):  # the entry launches on the current device
+    with on_device(dev):
         nat.check(nat.lib().rbp_results(found.data_ptr(), wfix.data_ptr(), B, int(stop_nconv), weights.data_ptr(), f64,
                                         valid.data_ptr(), u, u + 4 * B, torch.cuda.current_stream(dev).cuda_stream),
                   "rbp_results")
@@ -91,7 +101,7 @@ def queue_order(found: torch.Tensor, count: Optional[torch.Tensor] = None) -> to
     device of ``found`` and its current stream."""
     dev = found.device
     order = torch.empty(found.shape[0], dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):  # as above
+    with on_device(dev):
         nat.check(nat.lib().rbp_queue_order(found.data_ptr(), int(found.shape[0]), order.data_ptr(),
                                             count.data_ptr() if count is not None else None,
                                             torch.cuda.current_stream(dev).cuda_stream), "rbp_queue_order")

@@ -49,6 +49,7 @@ def calls(monkeypatch):
     library = Library()
     monkeypatch.setattr(nat, "lib", lambda: library)
     monkeypatch.setattr(torch.cuda, "device", Select)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: SimpleNamespace(cuda_stream=0))
     return log
 
