@@ -308,11 +308,21 @@ int choose_launch(int C, int V, int slots, int vslots, int rows, int msg_type, i
       return fail(RBP_ERR_UNSUPPORTED,
                   w + ": groups_per_block must be in [1, " + std::to_string(max_groups) + "] for this shape");
   }
-  const Layout L = fit_layout(C, V, rows, msg_type, G, vpt, NG, max_smem);
+  Layout L = fit_layout(C, V, rows, msg_type, G, vpt, NG, max_smem);
   RBP_CUDA(set_max_dynamic_smem(reinterpret_cast<const void*>(k), max_smem));
-  const size_t smem = block_fixed + (size_t)NG * L.group_bytes;
   int per_sm = 0;
-  RBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, G * NG, smem));
+  RBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, G * NG, block_fixed + (size_t)NG * L.group_bytes));
+  // The second resident block before the kept sums where only one of the two fits: the 2,000 x 4,000 code
+  // with 16-bit messages (83,392 B a block without the sums, 116,160 B with them), 60,000 shots at 256
+  // threads: one block with the sums 59.1 ms, two without 36.6 (512 threads, one block: 44.7).
+  if (blocks_per_sm == 2 && per_sm < 2 && L.sums) {
+    int without = 0;
+    RBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&without, k, G, block_fixed + (size_t)bare.group_bytes));
+    if (without >= 2) {
+      L = bare;
+      per_sm = without;
+    }
+  }
   if (per_sm < 1) return fail(RBP_ERR_UNSUPPORTED, w + ": launch shape has zero occupancy");
   *out = Launch{k, G, NG, per_sm * sm_count, nshots, blocks_per_sm, L};
   return RBP_OK;
