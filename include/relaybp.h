@@ -142,7 +142,8 @@ RBP_API int rbp_decoder_configure_kind(rbp_decoder* d, int32_t kind, int32_t gro
 
 /* Shared-memory bytes of one shot's region and of the block-wide tables for
  * the current message type; the RBP_LAUNCH_LEGS shape currently configured.
- * Any pointer may be NULL. */
+ * Where the library chooses, that is its shape for small batches
+ * (rbp_decoder_query_batch tells a batch's).  Any pointer may be NULL. */
 RBP_API int rbp_decoder_query(const rbp_decoder* d, int64_t* group_smem, int64_t* block_smem,
                       int32_t* group_threads, int32_t* groups_per_block, int32_t* blocks,
                       int32_t* shots_per_group);
@@ -153,6 +154,13 @@ RBP_API int rbp_decoder_query(const rbp_decoder* d, int64_t* group_smem, int64_t
 RBP_API int rbp_decoder_query_kind(const rbp_decoder* d, int32_t kind, int32_t* group_threads,
                                    int32_t* groups_per_block, int32_t* shots_per_group,
                                    int32_t* blocks_per_sm, int32_t* blocks);
+
+/* The shape a launch of that kind runs with for B shots: the configured one,
+ * or the library's own choice for a batch of that size.  Any pointer may be
+ * NULL. */
+RBP_API int rbp_decoder_query_batch(const rbp_decoder* d, int32_t kind, int64_t B, int64_t* group_smem,
+                                    int64_t* block_smem, int32_t* group_threads, int32_t* groups_per_block,
+                                    int32_t* shots_per_group, int32_t* blocks_per_sm, int32_t* blocks);
 
 /* Per-call inputs (device memory).  Optional pointers may be NULL.
  * Mirrors decode()'s keyword arguments (src/pelagos/decoder.py:2317-2361).

@@ -45,6 +45,7 @@ EXPORTED_SYMBOLS = (
     "rbp_decoder_query",
     "rbp_decoder_configure_kind",
     "rbp_decoder_query_kind",
+    "rbp_decoder_query_batch",
     "rbp_state_bytes",
     "rbp_state_posterior_offset",
     "rbp_decode",
@@ -183,6 +184,8 @@ def _declare(lib):
     lib.rbp_decoder_configure_kind.argtypes = [P, i32, i32, i32, i32, i32]
     lib.rbp_decoder_query_kind.restype = ct.c_int
     lib.rbp_decoder_query_kind.argtypes = [P, i32, i32p, i32p, i32p, i32p, i32p]
+    lib.rbp_decoder_query_batch.restype = ct.c_int
+    lib.rbp_decoder_query_batch.argtypes = [P, i32, i64, ct.POINTER(i64), ct.POINTER(i64), i32p, i32p, i32p, i32p, i32p]
     lib.rbp_state_bytes.restype = ct.c_int
     lib.rbp_state_bytes.argtypes = [P, ct.POINTER(i64)]
     lib.rbp_state_posterior_offset.restype = ct.c_int

@@ -75,6 +75,7 @@ struct rbp_decoder {
   int64_t bulk_from = INT64_MAX;     // batch size from which `bulk` runs
   int sm_count = 0;
   size_t max_smem = 0;
+  const Launch& shape_for(int k, int64_t B) const { return automatic[k] && B >= bulk_from ? bulk : shape[k]; }
 };
 
 namespace {
@@ -761,6 +762,23 @@ int rbp_decoder_query_kind(const rbp_decoder* d, int32_t kind, int32_t* group_th
   return RBP_OK;
 }
 
+int rbp_decoder_query_batch(const rbp_decoder* d, int32_t kind, int64_t B, int64_t* group_smem, int64_t* block_smem,
+                            int32_t* group_threads, int32_t* groups_per_block, int32_t* shots_per_group,
+                            int32_t* blocks_per_sm, int32_t* blocks) {
+  if (!d) return fail(RBP_ERR_ARGUMENT, "rbp_decoder_query: null decoder");
+  if (kind != RBP_LAUNCH_PRE && kind != RBP_LAUNCH_LEGS)
+    return fail(RBP_ERR_ARGUMENT, "rbp_decoder_query: kind must be RBP_LAUNCH_PRE or RBP_LAUNCH_LEGS");
+  const Launch& sh = d->shape_for(kind == RBP_LAUNCH_PRE ? 0 : 1, B);
+  if (group_smem) *group_smem = sh.L.group_bytes;
+  if (block_smem) *block_smem = sh.L.off_group0;
+  if (group_threads) *group_threads = sh.group_threads;
+  if (groups_per_block) *groups_per_block = sh.groups;
+  if (shots_per_group) *shots_per_group = sh.nshots;
+  if (blocks_per_sm) *blocks_per_sm = sh.minb;
+  if (blocks) *blocks = sh.blocks;
+  return RBP_OK;
+}
+
 int rbp_decode(rbp_decoder* d, int64_t B, const rbp_batch* in, const rbp_outputs* out, void* stream) {
   if (!d || !in || !out) return fail(RBP_ERR_ARGUMENT, "rbp_decode: null argument");
   int rc = check_batch("rbp_decode", B, in, out, d->p, d->n_alpha);
@@ -769,8 +787,7 @@ int rbp_decode(rbp_decoder* d, int64_t B, const rbp_batch* in, const rbp_outputs
   DeviceGuard dg(g->device);
   if (!dg.ok) return fail(RBP_ERR_CUDA, "rbp_decode: cannot select the CUDA device");
   // a launch that skips the relay legs runs at most pre_iter iterations per shot
-  const int k = in->skip_relay_legs ? 0 : 1;
-  const Launch& sh = d->automatic[k] && B >= d->bulk_from ? d->bulk : d->shape[k];
+  const Launch& sh = d->shape_for(in->skip_relay_legs ? 0 : 1, B);
   return launch_decode(device_graph(*d), d->p, sh, d->llr.p, d->gamma_legs.p, d->alpha.p, d->strict, d->queue.p, B, in,
                        out, reinterpret_cast<cudaStream_t>(stream), "rbp_decode");
 }

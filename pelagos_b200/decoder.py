@@ -142,23 +142,26 @@ class _NativeDecoder:
                                                        int(groups_per_block), int(shots_per_group),
                                                        int(blocks_per_sm)), "rbp_decoder_configure")
 
-    def query(self) -> dict:
+    def query(self, shots: Optional[int] = None) -> dict:
+        L = nat.lib()
         gs, bs = ct.c_int64(), ct.c_int64()
-        gt, gb, nb, ns = ct.c_int32(), ct.c_int32(), ct.c_int32(), ct.c_int32()
-        nat.check(nat.lib().rbp_decoder_query(self._dec, ct.byref(gs), ct.byref(bs), ct.byref(gt),
-                                              ct.byref(gb), ct.byref(nb), ct.byref(ns)), "rbp_decoder_query")
-        out = {"group_smem": gs.value, "block_smem": bs.value, "group_threads": gt.value,
-               "groups_per_block": gb.value, "blocks": nb.value, "shots_per_group": ns.value}
-        for kind, key in ((nat.RBP_LAUNCH_LEGS, None), (nat.RBP_LAUNCH_PRE, "pre")):
-            gt, gb, ns, bps, nb = (ct.c_int32() for _ in range(5))
-            nat.check(nat.lib().rbp_decoder_query_kind(self._dec, kind, ct.byref(gt), ct.byref(gb), ct.byref(ns),
-                                                       ct.byref(bps), ct.byref(nb)), "rbp_decoder_query")
-            if key is None:
-                out["blocks_per_sm"] = bps.value
+
+        def shape(kind):
+            v = {k: ct.c_int32() for k in ("group_threads", "groups_per_block", "shots_per_group", "blocks_per_sm",
+                                           "blocks")}
+            refs = [ct.byref(x) for x in v.values()]
+            if shots is None:
+                nat.check(L.rbp_decoder_query_kind(self._dec, kind, *refs), "rbp_decoder_query")
             else:
-                out[key] = {"group_threads": gt.value, "groups_per_block": gb.value, "shots_per_group": ns.value,
-                            "blocks_per_sm": bps.value, "blocks": nb.value}
-        return out
+                sizes = (ct.byref(gs), ct.byref(bs)) if kind == nat.RBP_LAUNCH_LEGS else (None, None)
+                nat.check(L.rbp_decoder_query_batch(self._dec, kind, int(shots), *sizes, *refs), "rbp_decoder_query")
+            return {k: x.value for k, x in v.items()}
+
+        legs = shape(nat.RBP_LAUNCH_LEGS)
+        if shots is None:
+            nat.check(L.rbp_decoder_query(self._dec, ct.byref(gs), ct.byref(bs), None, None, None, None),
+                      "rbp_decoder_query")
+        return {"group_smem": gs.value, "block_smem": bs.value, **legs, "pre": shape(nat.RBP_LAUNCH_PRE)}
 
     def decode(self, B: int, batch: nat.RbpBatch, outs: nat.RbpOutputs, stream: int):
         nat.check(nat.lib().rbp_decode(self._dec, int(B), ct.byref(batch), ct.byref(outs),
@@ -461,8 +464,11 @@ class RelayBPDecoder:
                 self._pre_launch = self._launch if self._launch is not None else (0, 0, 0, 0)
             self._launch = shape
 
-    def launch_info(self) -> dict:
-        return self._native[self.device_ids[0]].query()
+    def launch_info(self, shots: Optional[int] = None) -> dict:
+        """The configured launch shape (the pre-iteration launches' under ``"pre"``).  Where the library chooses,
+        it depends on the batch: ``shots`` gives that of a launch of so many shots, without it the shape of
+        small batches."""
+        return self._native[self.device_ids[0]].query(shots)
 
     def override_llr_columns(self, cols, value):
         """Overwrite prior LLRs (and selection weights) of some columns; returns a restore callable.

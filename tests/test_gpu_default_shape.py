@@ -37,3 +37,23 @@ def test_two_blocks_per_sm_come_before_the_kept_sums(dtype, per_sm):
     got = dec.decode(syn, return_last_posterior=True)  # results do not depend on the shape
     for k in ("errors", "weights", "valid_mask", "iterations", "found_count", "last_posterior"):
         assert torch.equal(got[k], want[k]), k
+
+
+# the message types of one code on either side of the batch size where the library's shape changes: 16 shots per
+# resident block of the second one
+@pytest.mark.parametrize("make,dtype,small,bulk", [
+    (lambda: codes.bb_phenomenological_144(12), "float32", (864, 1, 1), (448, 1, 2)),
+    (lambda: codes.bb_phenomenological_144(12), "bfloat16", (864, 1, 1), (448, 1, 2)),
+    (lambda: codes.regular_ldpc(C=2000, V=4000, seed=3), "float16", (512, 1, 1), (256, 1, 2)),
+    (lambda: codes.regular_ldpc(C=2000, V=4000, seed=3), "float32", (512, 1, 1), None),
+])
+def test_reported_shape_is_that_of_the_batch(make, dtype, small, bulk):
+    dec = _decoder(make(), dtype)
+    n = 16 * 2 * _sms()
+    keys = ("group_threads", "groups_per_block", "blocks_per_sm")
+    for shots, want in ((None, small), (n - 1, small), (n, bulk or small)):
+        info = dec.launch_info(shots)
+        assert tuple(info[k] for k in keys) == want, shots
+        assert tuple(info["pre"][k] for k in keys) == want, shots
+    dec.configure_launch(512, 1)  # an explicit shape holds for every batch
+    assert dec.launch_info(n) == dec.launch_info(1) == dec.launch_info()
