@@ -329,6 +329,53 @@ int choose_launch(int C, int V, int slots, int vslots, int rows, int msg_type, i
   return RBP_OK;
 }
 
+// The shape for large batches of a code of at most 2,048 variables, and the shots per resident group from which
+// it runs (0: the small batches' shape runs at every size).  A small batch waits for its slowest shots, so its
+// shape gives a shot as many threads as shorten one iteration; a large one waits for the SMs' issue slots, and
+// then fewer warps per shot, each with more variables, spend fewer of them on barriers, loop control and idle
+// lanes.  us with the small batches' shape / this one, 1,000,000 shots, float32:
+//   V    144  216  432  600  648  864  1,080  1,200  1,728
+//      29,914 27,586 58,258 76,140 67,293 66,534 91,392 180,849 121,755
+//      23,030 18,717 31,335 58,831 45,172 45,121 72,121 148,502 107,753
+// and 65,536 shots: 1,080 variables 7,687 / 8,275, 1,728 variables 11,453 / 12,228, since the slowest shot's
+// 6,080 iterations decide there.  From 224 shots per resident group (99,000 to 530,000 shots) on none loses: 150,000
+// shots of 1,080 variables 14,167 / 12,054, 400,000 of 216 variables 11,195 / 10,228.  Variables of more than
+// three edges keep the small batches' shape: at four variables per thread the kernel for two blocks per SM
+// spills their edge offsets.
+//  * V <= 96: one warp per shot, which needs no barrier, from 4 shots per group on: [[72,12,6]], 65,536 shots 964
+//    against 1,171, 8,192 shots 523 against 419.  (That is the one code it was set for; 85 variables of a
+//    repetition code, whose hard shots are more, 65,536 shots 10,059 against 8,023, 300,000 21,668 against 27,554.)
+//  * float64 holds twice the registers, and the kernel for two blocks per SM spills them from three variables per
+//    thread on.  Up to 512 variables it takes two per thread where that still covers the checks in one round, beyond
+//    that several groups per block of four (V <= 1,024) or eight: 300,000 shots 432 variables 25,099 / 17,971,
+//    648 variables 32,263 / 28,086, 1,080 variables 51,010 / 43,307, 1,728 variables 109,821 / 73,203; 150,000 shots of
+//    1,080 variables 26,080 / 27,827, so from 512 shots per group.
+int64_t choose_bulk(int C, int V, int slots, int vslots, int rows, int msg_type, size_t max_smem, int sm_count,
+                    const Launch& small, Launch* bulk, const char* who) {
+  const bool f64 = msg_type == RBP_MSG_F64;
+  int vpt, groups = 1, per_group = f64 ? 512 : 224;
+  if (f64 && V <= 512) {
+    vpt = 2;
+    per_group = V <= 96 ? 8 : 256;
+  } else if (f64) {
+    vpt = V <= 1024 ? 4 : 8;
+    groups = 0;
+  } else if (V <= 96) {
+    vpt = 3;
+    per_group = 4;
+  } else {
+    if (vslots > 3) return 0;
+    vpt = V <= 400 ? 3 : (V <= 1200 ? 4 : 6);
+  }
+  const int G = std::max(32, (V + vpt - 1) / vpt + 31) / 32 * 32;
+  if (groups == 1 && (G == small.group_threads || (f64 && G < C))) return 0;
+  if (choose_launch(C, V, slots, vslots, rows, msg_type, G, groups, max_smem, sm_count, bulk, who, 1,
+                    groups == 1 ? 2 : 1) != RBP_OK)
+    return 0;
+  if (groups == 1 && bulk->blocks < 2 * sm_count) return 0;
+  return (int64_t)per_group * bulk->blocks * bulk->groups;
+}
+
 // The library's own choice of shape: `small` for batches below `bulk_from`, `bulk` from there on.
 //
 // One group per block, compiled for two resident blocks per SM, with the fewest owned
@@ -339,12 +386,10 @@ int choose_launch(int C, int V, int slots, int vslots, int rows, int msg_type, i
 // seeds) against 2,242; 216 variables 65,536 shots 4,714 against 7,198; 648 variables 30,000 shots
 // 5,417 against 7,393; 1,728 variables 30,000 shots 6,721 against 8,990; [[72,12,6]] 100 shots 206
 // against 303.  A few more threads where they save a round of check rows (432 rows of 1,080
-// variables: 448 threads 6,125, 384 threads 6,567).  Two exceptions:
-//  * beyond four variables per thread (V > 2,048) a lone shot is no faster than with the
-//    other rule's larger group (2,592 variables, 2,000 shots: 4,622 against 4,530), so that one
-//    keeps batches of up to 16 shots per resident group; 65,536 shots: 15,300 against 20,200;
-//  * groups of one warp (V <= 96) need no barrier and win once they are four times
-//    oversubscribed: [[72,12,6]], 65,536 shots 964 against 1,171, but 8,192 shots 523 against 419.
+// variables: 448 threads 6,125, 384 threads 6,567).  Large batches: choose_bulk.  Beyond four variables
+// per thread (V > 2,048) a lone shot is no faster than with the other rule's larger group (2,592 variables,
+// 2,000 shots: 4,622 against 4,530), so that one keeps batches of up to 16 shots per resident group; 65,536
+// shots of 2,592 variables 15,300 against 20,200, 6,000 of 2,200 variables 3,250 against about 3,580.
 // A code whose blocks do not fit twice on an SM keeps the other rule.
 int choose_automatic(int C, int V, int slots, int vslots, int rows, int msg_type, size_t max_smem, int sm_count,
                      Launch* small, Launch* bulk, int64_t* bulk_from, const char* who) {
@@ -374,8 +419,13 @@ int choose_automatic(int C, int V, int slots, int vslots, int rows, int msg_type
       *bulk_from = 16LL * two.blocks;
       break;
     }
-    *small = two;
-    if (V <= 96 && two_per_sm(32, bulk)) *bulk_from = 4LL * bulk->blocks;
+    if (two.L.sums) {
+      *small = two;
+    } else if (const int rc = other_rule()) {  // without the kept sums a leg's first iteration takes longer
+      return rc;
+    }
+    const int64_t from = choose_bulk(C, V, slots, vslots, rows, msg_type, max_smem, sm_count, *small, bulk, who);
+    if (from > 0) *bulk_from = from;
     return RBP_OK;
   }
   return other_rule();

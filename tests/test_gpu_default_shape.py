@@ -57,3 +57,40 @@ def test_reported_shape_is_that_of_the_batch(make, dtype, small, bulk):
         assert tuple(info["pre"][k] for k in keys) == want, shots
     dec.configure_launch(512, 1)  # an explicit shape holds for every batch
     assert dec.launch_info(n) == dec.launch_info(1) == dec.launch_info()
+
+
+# large batches of codes of at most 2,048 variables: shots per resident group from which their shape runs, and
+# (threads, groups per block, blocks per SM) below and from there
+@pytest.mark.parametrize("make,dtype,per_group,small,bulk", [
+    (codes.bb_code_capacity_144, "float32", 224, (160, 1, 2), (64, 1, 2)),
+    (lambda: codes.bb_phenomenological_144(2), "float16", 224, (448, 1, 2), (128, 1, 2)),
+    (lambda: codes.bb_phenomenological_144(3), "bfloat16", 224, (352, 1, 2), (192, 1, 2)),
+    (lambda: codes.bb_phenomenological_144(8), "float32", 224, (448, 1, 2), (288, 1, 2)),
+    (codes.bb_code_capacity_72, "float64", 8, (96, 1, 2), (64, 1, 2)),
+    (lambda: codes.bb_phenomenological_144(2), "float64", 256, (448, 1, 2), (224, 1, 2)),
+    (lambda: codes.bb_phenomenological_144(3), "float64", 512, (352, 1, 2), (192, 4, 1)),
+    (lambda: codes.bb_phenomenological_144(8), "float64", 512, (576, 1, 1), (224, 2, 1)),
+])
+def test_large_batches_of_small_codes(make, dtype, per_group, small, bulk):
+    H = make()
+    dec = _decoder(H, dtype)
+    keys = ("group_threads", "groups_per_block", "blocks_per_sm")
+    n = 1 << 30
+    info = dec.launch_info(n)
+    assert tuple(info[k] for k in keys) == bulk
+    n = per_group * info["blocks"] * info["groups_per_block"]
+    assert tuple(dec.launch_info(n - 1)[k] for k in keys) == small
+    assert tuple(dec.launch_info(n)[k] for k in keys) == bulk
+    # the batch at the change, every result equal to another shape's (results do not depend on the shape)
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    A = torch.from_numpy(H.toarray().T.astype(np.float32)).to(DEV)
+    syn = torch.empty(n, H.shape[0], dtype=torch.uint8, device=DEV)
+    for i in range(0, n, 65536):
+        e = torch.rand(min(65536, n - i), H.shape[1], generator=gen, device=DEV) < 0.012
+        syn[i:i + 65536] = torch.remainder(e.float() @ A, 2).to(torch.uint8)
+    got = dec.decode(syn)
+    dec.configure_launch(*small[:2], 1, small[2])
+    want = dec.decode(syn)
+    for k in ("errors", "weights", "valid_mask", "iterations", "found_count"):
+        assert torch.equal(got[k], want[k]), k
+
