@@ -230,10 +230,11 @@ int vpt_for(int V, int G) {
   return -1;
 }
 
-// Default shape: the fewest owned variables per thread (from 3 up) whose group
+// Default shape: the fewest owned variables per thread (from `least` up) whose group
 // still fits the register budget of that count, so a shot's iteration is short.
-int default_group_threads(int C, int V, int nshots = 1, int minb = 1) {
+int default_group_threads(int C, int V, int nshots = 1, int minb = 1, int least = 3) {
   for (int vpt : {3, 4, 6, 8, 12, 16}) {
+    if (vpt < least) continue;
     const int G = std::max(32, (V + vpt - 1) / vpt + 31) / 32 * 32;
     if (G <= max_group_threads(vpt, nshots, minb) && (C + G - 1) / G <= 32 && vpt_for(V, G) <= vpt) return G;
   }
@@ -390,13 +391,17 @@ int64_t choose_bulk(int C, int V, int slots, int vslots, int rows, int msg_type,
 // per thread (V > 2,048) a lone shot is no faster than with the other rule's larger group (2,592 variables,
 // 2,000 shots: 4,622 against 4,530), so that one keeps batches of up to 16 shots per resident group; 65,536
 // shots of 2,592 variables 15,300 against 20,200, 6,000 of 2,200 variables 3,250 against about 3,580.
-// A code whose blocks do not fit twice on an SM keeps the other rule.
+// A code whose blocks do not fit twice on an SM keeps the other rule, with float64 messages and more than 2,048
+// variables from six variables per thread on (three spill): 2,592 variables, 864 / 448 threads, one shot 125 / 116,
+// 3,000 shots 7,900 / 7,707, 200,000 118,322 / 102,765; 2,200 variables, 736 / 384 threads, 242 / 227, 3,543 / 3,265,
+// 222,259 / 205,469; 3,000 variables, 768 / 512 threads, 282 / 253, 4,675 / 4,231, 294,253 / 266,205.
 int choose_automatic(int C, int V, int slots, int vslots, int rows, int msg_type, size_t max_smem, int sm_count,
                      Launch* small, Launch* bulk, int64_t* bulk_from, const char* who) {
   *bulk_from = INT64_MAX;
   auto other_rule = [&]() {
-    return choose_launch(C, V, slots, vslots, rows, msg_type, default_group_threads(C, V), 0, max_smem, sm_count, small,
-                         who);
+    const int least = msg_type == RBP_MSG_F64 && V > 2048 ? 6 : 3;
+    return choose_launch(C, V, slots, vslots, rows, msg_type, default_group_threads(C, V, 1, 1, least), 0, max_smem,
+                         sm_count, small, who);
   };
   auto two_per_sm = [&](int G, Launch* out) {
     return choose_launch(C, V, slots, vslots, rows, msg_type, G, 1, max_smem, sm_count, out, who, 1, 2) == RBP_OK &&

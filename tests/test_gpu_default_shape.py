@@ -94,3 +94,8 @@ def test_large_batches_of_small_codes(make, dtype, per_group, small, bulk):
     for k in ("errors", "weights", "valid_mask", "iterations", "found_count"):
         assert torch.equal(got[k], want[k]), k
 
+
+@pytest.mark.parametrize("V,threads", [(2200, 384), (3000, 512)])
+def test_float64_codes_above_2048_variables(V, threads):
+    info = _decoder(codes.regular_ldpc(C=V // 2, V=V, seed=3), "float64").launch_info()
+    assert (info["group_threads"], info["groups_per_block"], info["blocks_per_sm"]) == (threads, 1, 1)
