@@ -62,3 +62,12 @@ def test_failure_counts_match_the_general_products(B, N, R, offset):
     # int64 counts take the general products
     other = mc.failures(e, {"errors": est, "found_count": found.long(), "iterations": iters.long()})
     np.testing.assert_array_equal(other.cpu().numpy(), want)
+
+
+# rows read by column: tiles of 9, 17 and 32 shots with a partial last one, odd and 4-byte rows, a warp and a
+# thread per matrix row, one and four bytes per store
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("B,N,R", [(5323, 101, 70), (5323, 100, 63), (10001, 37, 5), (19003, 36, 68), (1900, 20001, 65)])
+def test_rows_read_by_column(B, N, R, offset):
+    test_matches_integer_product(B, N, R, offset)
+    test_failure_counts_match_the_general_products(B, N, R, offset)
