@@ -5,12 +5,18 @@
 // (src/pelagos/decoder.py:3839-3873); so did this library's.  Each is a launch of 2-3 us
 // on the device and 4-5 us on the host, a dozen of them and a radix sort per call: more
 // than the decode of a small batch.  Here each is one launch.  What bounds them is the
-// latency of one block's walk over the counts (ordered compaction), about 1,000 cycles
-// per 4,096 shots; the rest of a launch's blocks make the elementwise results beside it.
+// latency of the ordered compaction, a block's rounds of 16,384 counts (a warp takes 512,
+// loads and stores contiguous, ranks from ballots); the rest of a launch's blocks make the
+// elementwise results beside it.  From CLUSTER_FROM shots on a cluster of blocks shares the
+// walk: each takes a contiguous part, counts it, reads the others' counts from their shared
+// memory and compacts its own.  us per call, torch operations / one block for all in rounds of 4,096 /
+// now: order of 65,536 shots 87 / 45 / 22, of 1,048,576 97 / 498 / 63, of 4,194,304 157 / 1,947 / 205;
+// results 113 / 55 / 43, 111 / 223 / 64, 148 / 778 / 139.
 
 #include "relaybp.h"
 #include "relaybp_host.h"
 
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -19,32 +25,59 @@
 
 namespace {
 
+namespace cg = cooperative_groups;
 using rbph::fail;
 
-constexpr int FT = 1024;  // threads; the compacting block takes 4 FT shots per round
+constexpr int FT = 1024;  // threads
+constexpr int PER = 16;   // shots per thread in a compacting block's round
+constexpr int CLUSTER = 8;
+constexpr int64_t CLUSTER_FROM = 2 * PER * FT;  // below, one block has at most two rounds (16,384 shots: 2 us)
 
-// Counts i .. i+3 (past B: `pad`).
-__device__ __forceinline__ int4 load4(const int* found, long long i, long long B, int pad) {
-  if (i + 3 < B && (reinterpret_cast<uintptr_t>(found) & 15) == 0) return *reinterpret_cast<const int4*>(found + i);
-  int4 v = make_int4(pad, pad, pad, pad);
-  if (i < B) v.x = found[i];
-  if (i + 1 < B) v.y = found[i + 1];
-  if (i + 2 < B) v.z = found[i + 2];
-  if (i + 3 < B) v.w = found[i + 3];
-  return v;
+// The compacting blocks' parts of the B shots: whole rounds, so that loads stay aligned.
+struct Part {
+  long long i0, i1;
+};
+__device__ __forceinline__ Part part_of(long long B, unsigned rank, unsigned n) {
+  const long long rounds = (B + PER * FT - 1) / (PER * FT), each = (rounds + n - 1) / n * (PER * FT);
+  const long long i0 = min(B, each * rank);
+  return {i0, min(B, i0 + each)};
 }
 
-// Exclusive prefix sum of n over the block, and the block's total in *total.
-__device__ __forceinline__ int block_scan(int n, int* warp_sum, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int s = n;
+// A warp's PER x 32 counts of a round: bit l of below[k] tells whether found[i + 32 k + l] < limit (past the
+// part's end: not), i the warp's first shot.  The loads are contiguous and all in flight; returns the bits' number.
+__device__ __forceinline__ int load_round(const int* found, long long i, long long end, int limit, uint32_t (&below)[PER]) {
+  int v[PER], n = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, s, o);
-    if (lane >= o) s += t;
+  for (int k = 0; k < PER; ++k) {
+    const long long at = i + 32 * k + (threadIdx.x & 31);
+    v[k] = at < end ? found[at] : limit;
   }
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    below[k] = __ballot_sync(0xffffffffu, v[k] < limit);
+    n += __popc(below[k]);
+  }
+  return n;
+}
+
+// Number of found[i] < limit in the part (valid in every thread).
+__device__ __forceinline__ int count_below(const int* found, Part p, int limit, int* counter) {
+  if (threadIdx.x == 0) *counter = 0;
+  __syncthreads();
+  int mine = 0;
+  uint32_t below[PER];
+  for (long long i = p.i0 + (threadIdx.x >> 5) * (32 * PER); i < p.i1; i += PER * FT)
+    mine += load_round(found, i, p.i1, limit, below);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(counter, mine);
+  __syncthreads();
+  return *counter;
+}
+
+// Exclusive prefix sum of the warps' n, and the block's total in *total.
+__device__ __forceinline__ int warps_scan(int n, int* warp_sum, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __syncthreads();  // the last round's sums have been read
-  if (lane == 31) warp_sum[warp] = s;
+  if (lane == 0) warp_sum[warp] = n;
   __syncthreads();
   const int w = warp_sum[lane];  // FT / 32 = 32 warps
   int ws = w;
@@ -54,16 +87,34 @@ __device__ __forceinline__ int block_scan(int n, int* warp_sum, int* total) {
     if (lane >= o) ws += t;
   }
   *total = __shfl_sync(0xffffffffu, ws, 31);
-  return s - n + __shfl_sync(0xffffffffu, ws - w, warp);
+  return __shfl_sync(0xffffffffu, ws - w, warp);
 }
 
-// Block 0: the indices of shots with found < stop_nconv in ascending order, and their number.
+// The cluster's counts of the parts before this block's, and of all parts in *all.  A cluster of one
+// block needs neither.
+__device__ __forceinline__ int cluster_base(const cg::cluster_group& cluster, int* counter, int* all) {
+  cluster.sync();  // every block's counter is final
+  int before = 0, sum = 0;
+  const unsigned rank = cluster.block_rank();
+  for (unsigned r = 0; r < cluster.num_blocks(); ++r) {
+    const int c = *cluster.map_shared_rank(counter, r);
+    before += r < rank ? c : 0;
+    sum += c;
+  }
+  cluster.sync();  // no block leaves while another reads its counter
+  *all = sum;
+  return before;
+}
+
+// The first cluster: the indices of shots with found < stop_nconv in ascending order, and their number.
 // Other blocks: weights from the exact fixed-point weight (2^-32 units; +inf where there is
 // none) and the mask found >= stop_nconv.
 __global__ void __launch_bounds__(FT) results_kernel(const int* found, const long long* wfix, long long B, int S,
                                                      float* w32, double* w64, uint8_t* valid, int* idx, int* count) {
-  if (blockIdx.x > 0) {
-    const long long i = (blockIdx.x - 1) * (long long)FT + threadIdx.x;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const unsigned n = cluster.num_blocks();
+  if (blockIdx.x >= n) {
+    const long long i = (blockIdx.x - n) * (long long)FT + threadIdx.x;
     if (i >= B) return;
     const long long w = wfix[i];
     const double x = w == LLONG_MAX ? __longlong_as_double(0x7ff0000000000000ll)
@@ -74,55 +125,68 @@ __global__ void __launch_bounds__(FT) results_kernel(const int* found, const lon
     return;
   }
   __shared__ int warp_sum[32];
-  int base = 0;
-  for (long long i0 = 0; i0 < B; i0 += 4 * FT) {
-    const long long i = i0 + 4 * threadIdx.x;
-    const int4 f = load4(found, i, B, S);
-    const int n = (f.x < S) + (f.y < S) + (f.z < S) + (f.w < S);
-    int total;
-    int at = base + block_scan(n, warp_sum, &total);
-    if (f.x < S) idx[at++] = (int)i;
-    if (f.y < S) idx[at++] = (int)i + 1;
-    if (f.z < S) idx[at++] = (int)i + 2;
-    if (f.w < S) idx[at++] = (int)i + 3;
+  __shared__ int counter;
+  const Part p = part_of(B, blockIdx.x, n);
+  int base = 0, all = 0;  // such shots before this block's part, then before the round
+  if (n > 1) {
+    count_below(found, p, S, &counter);
+    base = cluster_base(cluster, &counter, &all);
+  }
+  const int lane = threadIdx.x & 31;
+  for (long long i0 = p.i0; i0 < p.i1; i0 += PER * FT) {
+    const long long i = i0 + (threadIdx.x >> 5) * (32 * PER);
+    uint32_t below[PER];
+    int total, at = base + warps_scan(load_round(found, i, p.i1, S, below), warp_sum, &total);
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      if (below[k] >> lane & 1u) idx[at + __popc(below[k] & ((1u << lane) - 1u))] = (int)i + 32 * k + lane;
+      at += __popc(below[k]);
+    }
     base += total;
   }
-  if (threadIdx.x == 0) *count = base;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *count = n > 1 ? all : base;
 }
 
 // Shots without a solution first, each part in ascending order, and the number of the former.
 __global__ void __launch_bounds__(FT) order_kernel(const int* found, long long B, int* order, int* count) {
+  const cg::cluster_group cluster = cg::this_cluster();
   __shared__ int warp_sum[32];
-  __shared__ int unsolved;
-  if (threadIdx.x == 0) unsolved = 0;
-  __syncthreads();
-  int mine = 0;
-#pragma unroll 4
-  for (long long i = 4 * threadIdx.x; i < B; i += 4 * FT) {
-    const int4 f = load4(found, i, B, 1);
-    mine += (f.x <= 0) + (f.y <= 0) + (f.z <= 0) + (f.w <= 0);
-  }
-  mine = __reduce_add_sync(0xffffffffu, mine);
-  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&unsolved, mine);
-  __syncthreads();
-  const int first = unsolved;
-  int base = 0;  // unsolved shots before this round
-  for (long long i0 = 0; i0 < B; i0 += 4 * FT) {
-    const long long i = i0 + 4 * threadIdx.x;
-    const int4 f = load4(found, i, B, 1);
-    const int n = (f.x <= 0) + (f.y <= 0) + (f.z <= 0) + (f.w <= 0);
-    int total;
-    int u = base + block_scan(n, warp_sum, &total);  // unsolved before shot i
-    const int v[4] = {f.x, f.y, f.z, f.w};
+  __shared__ int counter;
+  const Part p = part_of(B, blockIdx.x, cluster.num_blocks());
+  int first = count_below(found, p, 1, &counter);  // unsolved shots of the batch
+  int base = 0;                                    // unsolved shots before the round
+  if (cluster.num_blocks() > 1) base = cluster_base(cluster, &counter, &first);
+  const int lane = threadIdx.x & 31;
+  for (long long i0 = p.i0; i0 < p.i1; i0 += PER * FT) {
+    const long long i = i0 + (threadIdx.x >> 5) * (32 * PER);
+    uint32_t below[PER];
+    int total, u = base + warps_scan(load_round(found, i, p.i1, 1, below), warp_sum, &total);  // unsolved before shot i
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (i + k >= B) break;
-      if (v[k] <= 0) order[u++] = (int)i + k;
-      else order[first + (int)i + k - u] = (int)i + k;
+    for (int k = 0; k < PER; ++k) {
+      const int shot = (int)i + 32 * k + lane, before = u + __popc(below[k] & ((1u << lane) - 1u));
+      if (below[k] >> lane & 1u) order[before] = shot;
+      else if (i + 32 * k + lane < p.i1) order[first + shot - before] = shot;
+      u += __popc(below[k]);
     }
     base += total;
   }
-  if (threadIdx.x == 0 && count) *count = first;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && count) *count = first;
+}
+
+// `blocks` blocks in clusters of `cluster`.
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), int blocks, int cluster, cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(FT);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 }  // namespace
@@ -134,20 +198,21 @@ int rbp_results(const int32_t* found_count, const int64_t* weight_fixed, int64_t
   if (B < 0 || B > INT_MAX) return fail(RBP_ERR_ARGUMENT, "rbp_results: batch out of range");
   if (!n_unconverged || (B > 0 && (!found_count || !weight_fixed || !weights || !valid || !unconverged)))
     return fail(RBP_ERR_ARGUMENT, "rbp_results: null buffer");
-  const int blocks = 1 + (int)((B + FT - 1) / FT);
-  results_kernel<<<blocks, FT, 0, static_cast<cudaStream_t>(stream)>>>(
-      found_count, reinterpret_cast<const long long*>(weight_fixed), B, stop_nconv,
-      weights_f64 ? nullptr : static_cast<float*>(weights), weights_f64 ? static_cast<double*>(weights) : nullptr, valid,
-      unconverged, n_unconverged);
-  RBP_CUDA(cudaGetLastError());
+  const int cluster = B < CLUSTER_FROM ? 1 : CLUSTER;
+  const int blocks = cluster + (int)(((B + FT - 1) / FT + cluster - 1) / cluster * cluster);
+  RBP_CUDA(launch(results_kernel, blocks, cluster, static_cast<cudaStream_t>(stream), found_count,
+                  reinterpret_cast<const long long*>(weight_fixed), (long long)B, (int)stop_nconv,
+                  weights_f64 ? nullptr : static_cast<float*>(weights), weights_f64 ? static_cast<double*>(weights) : nullptr,
+                  valid, unconverged, n_unconverged));
   return RBP_OK;
 }
 
 int rbp_queue_order(const int32_t* found_count, int64_t B, int32_t* order, int32_t* n_unsolved, void* stream) {
   if (B < 0 || B > INT_MAX) return fail(RBP_ERR_ARGUMENT, "rbp_queue_order: batch out of range");
   if (B > 0 && (!found_count || !order)) return fail(RBP_ERR_ARGUMENT, "rbp_queue_order: null buffer");
-  order_kernel<<<1, FT, 0, static_cast<cudaStream_t>(stream)>>>(found_count, B, order, n_unsolved);
-  RBP_CUDA(cudaGetLastError());
+  const int cluster = B < CLUSTER_FROM ? 1 : CLUSTER;
+  RBP_CUDA(launch(order_kernel, cluster, cluster, static_cast<cudaStream_t>(stream), found_count, (long long)B, order,
+                  n_unsolved));
   return RBP_OK;
 }
 
