@@ -74,7 +74,7 @@ HARD_FIRST_MIN_BATCH = 1024
 
 def on_device(device: torch.device):
     """Context in which ``device`` is the current one: native entries without a handle launch on the current
-    device.  Nothing to enter where it is already (0.3 us against 2 us for torch.cuda.device)."""
+    device.  Nothing to enter where it is already (asking takes 0.25 us, torch.cuda.device 1.5)."""
     if torch.cuda.current_device() == device.index:
         return nullcontext()
     return torch.cuda.device(device)
