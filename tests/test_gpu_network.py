@@ -89,3 +89,40 @@ def _check_gradients(size, B):
         a, b = got[o:o + n], ref[o:o + n]
         err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-12)
         assert err < 1e-2, f"{name}: relative gradient error {err:.3g}"
+
+
+@pytest.mark.parametrize("size", [s for s in SIZES if s[2] <= 8 and s[3] <= 4])
+def test_both_inference_kernels_give_the_same_bits(size):
+    """The low-degree kernel against the general one: a separate check of nine edges sends the same graph to the
+    general kernel and, sharing no variable with it, changes none of its values."""
+    H, dec, net, theta, syn, post = _setup(size, 77)
+    C, V = H.shape
+    wide = np.zeros((C + 1, V + 9), np.uint8)
+    wide[:C, :V] = H.toarray()
+    wide[C, V:] = 1
+    priors = np.concatenate([np.random.default_rng(7).uniform(0.01, 0.05, V), np.full(9, 0.02)])  # V as _setup draws them
+    dec2 = RelayBPDecoder(csr_matrix(wide), priors, algo="relay", pre_iter=5, num_sets=2, set_max_iter=5)
+    assert np.array_equal(dec2.log_prior_ratios[:V], dec.log_prior_ratios)
+    syn2 = np.concatenate([syn, np.ones((77, 1), np.uint8)], axis=1)
+    post2 = np.concatenate([post, np.full((77, 9), 3.0, np.float32)], axis=1)
+    gam, r = net.propose(*(torch.from_numpy(a).to(DEV) for a in (syn, post)), -0.24, 0.66, logits=True)
+    gam2, r2 = ProposalNet(dec2, theta).propose(*(torch.from_numpy(a).to(DEV) for a in (syn2, post2)), -0.24, 0.66,
+                                                 logits=True)
+    assert torch.equal(r, r2[:, :V].contiguous()) and torch.equal(gam, gam2[:, :V].contiguous())
+
+
+@pytest.mark.parametrize("B", [37, 1023, 1024])  # one row per thread, and two from 37,888 rows on
+def test_training_steps_repeat_bit_for_bit(B):
+    H, dec, _, theta, syn, post = _setup((37, 64, 8, 3), B)
+    target = np.random.default_rng(3).integers(0, 2, (B, H.shape[1])).astype(np.uint8)
+    args = [torch.from_numpy(a).to(DEV) for a in (syn, post, target)]
+    runs = []
+    for _ in range(3):
+        net = ProposalNet(dec, theta)
+        loss, grads = torch.zeros(1, device=DEV), torch.zeros(4805, device=DEV)
+        for _ in range(2):
+            net.train_step(*args, TrainConfig(), 1e-3, loss, grads)
+        runs.append((loss, grads, net.params()))
+    for other in runs[1:]:
+        for a, b in zip(runs[0], other):
+            assert torch.equal(a, b)
