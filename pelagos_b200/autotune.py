@@ -18,8 +18,8 @@ the reference keys its tuning cache (src/pelagos/autotune.py:130-133, 222-541):
 * candidates: every warp multiple G from 32 to 1024 that gives at most 16
   variables and 32 checks per thread, with several groups per block (the largest
   group count that fits and, for one-warp groups, also 8) and with one group
-  per block (at one resident block per SM, also in the two-shot form, and at
-  two);
+  per block, at one and at two resident blocks per SM (a shape of two shots per
+  group runs the kernel of one, so it is not timed again);
 * a candidate the library rejects (shared memory, registers) is skipped.
 
 ``default_shape`` returns the shape measured best for a workload and
@@ -80,18 +80,16 @@ def _store(key: str, value) -> None:
 
 def candidates(C: int, V: int) -> List[Tuple[int, int, int]]:
     out = []
-    for ns in (1, 2):
-        for G in range(32, 1025, 32):
-            need = -(-V // G)
-            if need > 16 or -(-C // G) > 32:
-                continue
-            if ns == 1:
-                out.append((G, 0, 1))   # several one-shot groups per block, as many as fit
-                if G == 32:
-                    out.append((G, 8, 1))
-            out.append((G, 1, ns))      # the block-per-group kernel
-            if ns == 1 and G <= 512:
-                out.append((G, 1, 1, 2))  # the same, compiled for two resident blocks per SM
+    for G in range(32, 1025, 32):
+        need = -(-V // G)
+        if need > 16 or -(-C // G) > 32:
+            continue
+        out.append((G, 0, 1))  # several groups per block, as many as fit
+        if G == 32:
+            out.append((G, 8, 1))
+        out.append((G, 1, 1))  # one group per block
+        if G <= 512:
+            out.append((G, 1, 1, 2))  # the same, compiled for two resident blocks per SM
     return out
 
 

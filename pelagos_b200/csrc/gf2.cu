@@ -24,6 +24,7 @@
 namespace {
 
 using rbph::fail;
+using rbph::kSMs;
 
 constexpr int GF2_THREADS = 256;
 constexpr int GF2_SHOTS = 32;  // shots per tile: the bits of a word
@@ -277,9 +278,9 @@ int launch_rows(const uint8_t* x, long long B, int N, const int* row_ptr, const 
                                   (int)smem));
   // whole words of shots once every SM has work for its resident blocks; small batches are
   // spread over the SMs instead
-  const long long spread = 148LL * 4;
+  const long long spread = 4LL * kSMs;
   const int tile = (int)std::min<long long>(GF2_SHOTS, std::max<long long>(1, (B + spread - 1) / spread));
-  const int blocks = (int)std::min<long long>((B + tile - 1) / tile, 148LL * 8);
+  const int blocks = (int)std::min<long long>((B + tile - 1) / tile, 8LL * kSMs);
   const int block = IN != STAGED && smem > WIDE_SMEM ? 2 * GF2_THREADS : GF2_THREADS;
   kernel<<<blocks, block, smem, st>>>(x, B, tile, N, piece_magic(N), row_ptr, cols, R, out);
   RBP_CUDA(cudaGetLastError());
@@ -353,9 +354,9 @@ int launch_failures(const uint8_t* e, const uint8_t* est, long long B, int N, co
   if (smem > 47 * 1024)
     RBP_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem));
-  const long long spread = 148LL * 4;
+  const long long spread = 4LL * kSMs;
   const int tile = (int)std::min<long long>(GF2_SHOTS, std::max<long long>(1, (B + spread - 1) / spread));
-  const int blocks = (int)std::min<long long>((B + tile - 1) / tile, 148LL * 8);
+  const int blocks = (int)std::min<long long>((B + tile - 1) / tile, 8LL * kSMs);
   const int block = IN != STAGED && smem > WIDE_SMEM ? 2 * GF2_THREADS : GF2_THREADS;
   RBP_CUDA(cudaMemsetAsync(counts, 0, 4 * sizeof(unsigned long long), st));
   kernel<<<blocks, block, smem, st>>>(e, est, B, tile, N, piece_magic(N), row_ptr, cols, R, found, iters, counts);

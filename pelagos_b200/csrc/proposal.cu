@@ -51,6 +51,7 @@ namespace {
 using rbph::DevBuf;
 using rbph::DeviceGuard;
 using rbph::fail;
+using rbph::kSMs;
 using bf16 = __nv_bfloat16;
 
 constexpr int NH = 64;   // node state width
@@ -168,7 +169,7 @@ __global__ void feat_var_kernel(NetGraph g, long long B, const uint8_t* syn, con
 // Gradients are summed in three steps: fp32 within a block (over its rows), one partial sum
 // per block in memory, and the blocks' sums in double.  With an atomic add per block the
 // additions to the running fp32 sum were the larger part of the error.
-constexpr int GRAD_BLOCKS = 148 * 4;               // at most so many blocks add to a parameter
+constexpr int GRAD_BLOCKS = kSMs * 4;               // at most so many blocks add to a parameter
 constexpr int GRAD_STRIDE = (N_PARAMS + 1 + 3) / 4 * 4;  // the loss comes after the parameters
 constexpr int RT = 128;       // threads (rows) of a row kernel's tile
 // Rows per thread of the row kernels: each weight read from shared memory serves that many rows.
@@ -176,7 +177,7 @@ constexpr int RT = 128;       // threads (rows) of a row kernel's tile
 // 191 (four rows: 108, 253, 266); backward stages 0-2 305, 250, 190 / 274, 240, 234.  So two,
 // one in the last of these, and one where two would leave SMs without a block: a step of 16
 // shots (14,976 rows) takes 141 us with one row and 156 with two, of 64 shots 246 and 237.
-constexpr unsigned TWO_ROWS_FROM = 148 * 2 * RT;
+constexpr unsigned TWO_ROWS_FROM = kSMs * 2 * RT;
 __host__ __device__ constexpr int forward_blocks(int rows) { return rows == 1 ? 6 : 4; }  // resident per SM
 __host__ __device__ constexpr int backward_blocks(int rows) { return rows == 1 ? 4 : 2; }
 constexpr int SY = NH + 4;    // padded shared-memory rows of the gradient tiles
@@ -1483,7 +1484,7 @@ __global__ void __launch_bounds__(PROPOSE_THREADS, 1) net_propose_fast_kernel(Ne
 
 int grid_for(long long n, int threads = 256) {
   const long long b = (n + threads - 1) / threads;
-  return (int)std::max(1LL, std::min(b, 148LL * 16));
+  return (int)std::max(1LL, std::min(b, 16LL * kSMs));
 }
 
 }  // namespace
@@ -1556,7 +1557,7 @@ struct rbp_net {
     const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
     // weights are staged once per block: the resident blocks loop over their rows
     const int R = rows_per_thread(nc);
-    const unsigned rows = std::min<unsigned>((nc + RT * R - 1) / (RT * R), 148 * forward_blocks(R));
+    const unsigned rows = std::min<unsigned>((nc + RT * R - 1) / (RT * R), kSMs * forward_blocks(R));
     const dim3 halves((nv + 255) / 256, 2);
     const bf16* t = theta_bf.p;
     feat_var_kernel<<<grid_for(nv), 256, 0, st>>>(g, B, syn, post, w.z, w.ty);
@@ -1573,7 +1574,7 @@ struct rbp_net {
     const NetWork& w = ws;
     const unsigned nc = (unsigned)(B * C), nv = (unsigned)(B * V);
     const dim3 quarters((nv + 255) / 256, 4);
-    const auto blocks = [&](int rows) { return (int)std::min<unsigned>((nc + RT * rows - 1) / (RT * rows), 148 * backward_blocks(rows)); };
+    const auto blocks = [&](int rows) { return (int)std::min<unsigned>((nc + RT * rows - 1) / (RT * rows), kSMs * backward_blocks(rows)); };
     const int R = rows_per_thread(nc), tiles = blocks(R), last = blocks(1);
     const int gather = (int)std::min<unsigned>((nc + 127) / 128, GRAD_BLOCKS);
     float* pg = partial;

@@ -161,7 +161,8 @@ KernelFn pick2_kernel(int msg_type, int dc, int dv, int vpt) {
   }
 }
 
-// Largest group that may be configured with two shots per group (the limits callers know).
+// Largest group that may be configured with two shots per group: the limits that shape always had, so that
+// what was refused stays refused.
 int max_two_shot_threads(int vpt) { return vpt <= 4 ? 512 : (vpt == 6 ? 480 : (vpt == 8 ? 384 : (vpt == 12 ? 256 : 192))); }
 
 int max_group_threads(int vpt, int nshots, int minb) {
@@ -480,7 +481,8 @@ bool strict_rows(const rbp_params& p, const float* alpha, int n_alpha) {
 
 // Fill the kernel arguments and launch (memset of the work counter + kernel) on `st`.
 int launch_decode(const DevGraph& dgph, const rbp_params& p, const Launch& lc, const float* llr,
-                  const float* gamma_legs, const float* alpha, bool strict, int* queue, int64_t B, const rbp_batch* in, const rbp_outputs* out, cudaStream_t st, const char* who) {
+                  const float* gamma_legs, const float* alpha, bool strict, int* queue, int64_t B, const rbp_batch* in,
+                  const rbp_outputs* out, cudaStream_t st, const char* who) {
   const Layout& L = lc.L;
   DevArgs a{};
   a.strict = strict;
@@ -530,7 +532,6 @@ int launch_decode(const DevGraph& dgph, const rbp_params& p, const Launch& lc, c
   a.off_chk_deg = L.off_chk_deg;
   a.off_llr = L.off_llr;
   a.off_first = L.off_first;
-  a.first_table = 1;
   a.off_group0 = L.off_group0;
   a.group_bytes = L.group_bytes;
   a.g_msg = L.g_msg;
@@ -920,7 +921,7 @@ int mixed_args(rbp_mixed* m, const int64_t* B, const rbp_batch* ins, const rbp_o
     a.solved_gamma = in->solved_gamma;
     a.solved_legs = in->solved_legs;
     a.suspend_unsolved = in->suspend_unsolved;
-      a.init_post = in->init_posterior;
+    a.init_post = in->init_posterior;
     a.errors = out->errors;
     a.errors_packed = out->errors_packed;
     a.weights = out->weights;
@@ -938,8 +939,7 @@ int mixed_args(rbp_mixed* m, const int64_t* B, const rbp_batch* ins, const rbp_o
     a.groups = m->NG[i];
     a.off_chk_deg = L.off_chk_deg;
     a.off_llr = L.off_llr;
-      a.off_first = L.off_first;
-    a.first_table = 1;
+    a.off_first = L.off_first;
     a.off_group0 = L.off_group0;
     a.group_bytes = L.group_bytes;
     a.g_msg = L.g_msg;

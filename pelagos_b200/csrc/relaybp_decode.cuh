@@ -134,7 +134,7 @@ __device__ __forceinline__ void run_group(const DevGraph& g, const DevArgs& a, u
   A* s1 = reinterpret_cast<A*>(region + a.g_s1);
   A* lmk = s1 + VPT * G;
 
-  const bool first_from_table = MAXDC > 0 && a.first_table && a.llr_shot == nullptr;
+  const bool first_from_table = MAXDC > 0 && a.llr_shot == nullptr;
   // the default rounding of the memory mix, shared priors, no offset and finite check outputs:
   // the steady loop without per-launch choices
   const bool usual = a.mix_mode == RBP_MIX_SEPARATE && a.llr_shot == nullptr && !a.use_beta && !a.strict;
@@ -662,7 +662,7 @@ template <typename M, int MAXDC>
 __device__ __forceinline__ void block_tables(const DevGraph& g, const DevArgs& a, unsigned char* smem) {
   load_block_tables(g, a, smem);
   __syncthreads();
-  if (a.first_table) build_first_pass_table<M, MAXDC>(g, a, smem);
+  build_first_pass_table<M, MAXDC>(g, a, smem);
 }
 
 // One code, one launch (rbp_decode, rbp_decode_static): a.groups groups per block.

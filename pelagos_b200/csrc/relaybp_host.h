@@ -39,6 +39,10 @@ struct DeviceGuard {
   }
 };
 
+// SMs of the only device these kernels are built for, where a grid's size is a matter of speed alone (the
+// decoder, whose shapes depend on it, asks the device).
+constexpr int kSMs = 148;
+
 inline int align16(int x) { return (x + 15) & ~15; }
 
 template <typename T>

@@ -102,21 +102,6 @@ __device__ __forceinline__ bool group_any(int id, int n, bool p) {
   return r != 0;
 }
 
-// Barrier + AND-reduction of a predicate over the group.
-__device__ __forceinline__ bool group_all(int id, int n, bool p) {
-  if (n == 32) return __all_sync(0xffffffffu, p);
-  unsigned r;
-  asm volatile(
-      "{\n\t.reg .pred pi, po;\n\t"
-      "setp.ne.u32 pi, %1, 0;\n\t"
-      "bar.red.and.pred po, %2, %3, pi;\n\t"
-      "selp.u32 %0, 1, 0, po;\n\t}"
-      : "=r"(r)
-      : "r"((unsigned)p), "r"(id), "r"(n)
-      : "memory");
-  return r != 0;
-}
-
 // ------------------------------------------------------------------ parameters
 
 struct DevGraph {
@@ -177,7 +162,6 @@ struct DevArgs {
   int group_threads, groups;
   // shared-memory layout (byte offsets)
   int off_chk_deg, off_llr, off_first, off_group0, group_bytes;
-  int first_table;               // 1: take each phase's first check pass from the block's table
   int g_msg, g_par, g_best, g_first, g_red;
   int keep_sums;                 // 1: the group region has the s1 and lmk arrays
   int g_s1;                      // the shot's first-pass sums, then the memory mixes
