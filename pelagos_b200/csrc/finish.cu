@@ -5,8 +5,8 @@
 // (src/pelagos/decoder.py:3839-3873); so did this library's.  Each is a launch of 2-3 us
 // on the device and 4-5 us on the host, a dozen of them and a radix sort per call: more
 // than the decode of a small batch.  Here each is one launch.  What bounds them is the
-// latency of the ordered compaction, a block's rounds of 16,384 counts (a warp takes 512,
-// loads and stores contiguous, ranks from ballots); the rest of a launch's blocks make the
+// latency of the ordered compaction, a block's rounds of up to 16,384 counts (a warp takes up to
+// 512, loads and stores contiguous, ranks from ballots); the rest of a launch's blocks make the
 // elementwise results beside it.  From CLUSTER_FROM shots on a cluster of blocks shares the
 // walk: each takes a contiguous part, counts it, reads the others' counts from their shared
 // memory and compacts its own.  us per call, torch operations / one block for all in rounds of 4,096 /
@@ -29,14 +29,19 @@ namespace cg = cooperative_groups;
 using rbph::fail;
 
 constexpr int FT = 1024;  // threads
-constexpr int PER = 16;   // shots per thread in a compacting block's round
 constexpr int CLUSTER = 8;
-constexpr int64_t CLUSTER_FROM = 2 * PER * FT;  // below, one block has at most two rounds (16,384 shots: 2 us)
+// Shots per thread in a compacting block's round (PER): few where one round takes the batch, since a round's
+// instructions are the time then (order / results on the device, one shot: 4 per thread 2.4 / 2.0 us, 16 per
+// thread 4.7 / 3.3; 16,384 shots 8.3 / 4.1 and 8.4 / 4.1; in a cluster 32,768 take 10.2 / 7.5, in one block 14.4 / 6.5).
+constexpr int PER_SMALL = 4, PER_LARGE = 16;
+constexpr int64_t LARGE_FROM = 2 * PER_SMALL * FT;
+constexpr int64_t CLUSTER_FROM = 2 * PER_LARGE * FT;
 
 // The compacting blocks' parts of the B shots: whole rounds, so that loads stay aligned.
 struct Part {
   long long i0, i1;
 };
+template <int PER>
 __device__ __forceinline__ Part part_of(long long B, unsigned rank, unsigned n) {
   const long long rounds = (B + PER * FT - 1) / (PER * FT), each = (rounds + n - 1) / n * (PER * FT);
   const long long i0 = min(B, each * rank);
@@ -45,7 +50,9 @@ __device__ __forceinline__ Part part_of(long long B, unsigned rank, unsigned n) 
 
 // A warp's PER x 32 counts of a round: bit l of below[k] tells whether found[i + 32 k + l] < limit (past the
 // part's end: not), i the warp's first shot.  The loads are contiguous and all in flight; returns the bits' number.
+template <int PER>
 __device__ __forceinline__ int load_round(const int* found, long long i, long long end, int limit, uint32_t (&below)[PER]) {
+  if (i >= end) return 0;  // the whole warp
   int v[PER], n = 0;
 #pragma unroll
   for (int k = 0; k < PER; ++k) {
@@ -61,13 +68,14 @@ __device__ __forceinline__ int load_round(const int* found, long long i, long lo
 }
 
 // Number of found[i] < limit in the part (valid in every thread).
+template <int PER>
 __device__ __forceinline__ int count_below(const int* found, Part p, int limit, int* counter) {
   if (threadIdx.x == 0) *counter = 0;
   __syncthreads();
   int mine = 0;
   uint32_t below[PER];
   for (long long i = p.i0 + (threadIdx.x >> 5) * (32 * PER); i < p.i1; i += PER * FT)
-    mine += load_round(found, i, p.i1, limit, below);
+    mine += load_round<PER>(found, i, p.i1, limit, below);
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(counter, mine);
   __syncthreads();
   return *counter;
@@ -109,6 +117,7 @@ __device__ __forceinline__ int cluster_base(const cg::cluster_group& cluster, in
 // The first cluster: the indices of shots with found < stop_nconv in ascending order, and their number.
 // Other blocks: weights from the exact fixed-point weight (2^-32 units; +inf where there is
 // none) and the mask found >= stop_nconv.
+template <int PER>
 __global__ void __launch_bounds__(FT) results_kernel(const int* found, const long long* wfix, long long B, int S,
                                                      float* w32, double* w64, uint8_t* valid, int* idx, int* count) {
   const cg::cluster_group cluster = cg::this_cluster();
@@ -126,41 +135,46 @@ __global__ void __launch_bounds__(FT) results_kernel(const int* found, const lon
   }
   __shared__ int warp_sum[32];
   __shared__ int counter;
-  const Part p = part_of(B, blockIdx.x, n);
+  const Part p = part_of<PER>(B, blockIdx.x, n);
   int base = 0, all = 0;  // such shots before this block's part, then before the round
   if (n > 1) {
-    count_below(found, p, S, &counter);
+    count_below<PER>(found, p, S, &counter);
     base = cluster_base(cluster, &counter, &all);
   }
   const int lane = threadIdx.x & 31;
   for (long long i0 = p.i0; i0 < p.i1; i0 += PER * FT) {
     const long long i = i0 + (threadIdx.x >> 5) * (32 * PER);
     uint32_t below[PER];
-    int total, at = base + warps_scan(load_round(found, i, p.i1, S, below), warp_sum, &total);
+    int total, at = base + warps_scan(load_round<PER>(found, i, p.i1, S, below), warp_sum, &total);
+    base += total;
+    if (i >= p.i1) continue;  // a warp without shots in the last round: its bits are not set
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       if (below[k] >> lane & 1u) idx[at + __popc(below[k] & ((1u << lane) - 1u))] = (int)i + 32 * k + lane;
       at += __popc(below[k]);
     }
-    base += total;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *count = n > 1 ? all : base;
 }
 
 // Shots without a solution first, each part in ascending order, and the number of the former.
+template <int PER>
 __global__ void __launch_bounds__(FT) order_kernel(const int* found, long long B, int* order, int* count) {
   const cg::cluster_group cluster = cg::this_cluster();
   __shared__ int warp_sum[32];
   __shared__ int counter;
-  const Part p = part_of(B, blockIdx.x, cluster.num_blocks());
-  int first = count_below(found, p, 1, &counter);  // unsolved shots of the batch
+  const Part p = part_of<PER>(B, blockIdx.x, cluster.num_blocks());
+  int first = count_below<PER>(found, p, 1, &counter);  // unsolved shots of the batch
   int base = 0;                                    // unsolved shots before the round
   if (cluster.num_blocks() > 1) base = cluster_base(cluster, &counter, &first);
   const int lane = threadIdx.x & 31;
   for (long long i0 = p.i0; i0 < p.i1; i0 += PER * FT) {
     const long long i = i0 + (threadIdx.x >> 5) * (32 * PER);
     uint32_t below[PER];
-    int total, u = base + warps_scan(load_round(found, i, p.i1, 1, below), warp_sum, &total);  // unsolved before shot i
+    int total;
+    int u = base + warps_scan(load_round<PER>(found, i, p.i1, 1, below), warp_sum, &total);  // unsolved before shot i
+    base += total;
+    if (i >= p.i1) continue;  // as above
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       const int shot = (int)i + 32 * k + lane, before = u + __popc(below[k] & ((1u << lane) - 1u));
@@ -168,7 +182,6 @@ __global__ void __launch_bounds__(FT) order_kernel(const int* found, long long B
       else if (i + 32 * k + lane < p.i1) order[first + shot - before] = shot;
       u += __popc(below[k]);
     }
-    base += total;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0 && count) *count = first;
 }
@@ -200,10 +213,10 @@ int rbp_results(const int32_t* found_count, const int64_t* weight_fixed, int64_t
     return fail(RBP_ERR_ARGUMENT, "rbp_results: null buffer");
   const int cluster = B < CLUSTER_FROM ? 1 : CLUSTER;
   const int blocks = cluster + (int)(((B + FT - 1) / FT + cluster - 1) / cluster * cluster);
-  RBP_CUDA(launch(results_kernel, blocks, cluster, static_cast<cudaStream_t>(stream), found_count,
-                  reinterpret_cast<const long long*>(weight_fixed), (long long)B, (int)stop_nconv,
-                  weights_f64 ? nullptr : static_cast<float*>(weights), weights_f64 ? static_cast<double*>(weights) : nullptr,
-                  valid, unconverged, n_unconverged));
+  RBP_CUDA(launch(B < LARGE_FROM ? results_kernel<PER_SMALL> : results_kernel<PER_LARGE>, blocks, cluster,
+                  static_cast<cudaStream_t>(stream), found_count, reinterpret_cast<const long long*>(weight_fixed),
+                  (long long)B, (int)stop_nconv, weights_f64 ? nullptr : static_cast<float*>(weights),
+                  weights_f64 ? static_cast<double*>(weights) : nullptr, valid, unconverged, n_unconverged));
   return RBP_OK;
 }
 
@@ -211,8 +224,8 @@ int rbp_queue_order(const int32_t* found_count, int64_t B, int32_t* order, int32
   if (B < 0 || B > INT_MAX) return fail(RBP_ERR_ARGUMENT, "rbp_queue_order: batch out of range");
   if (B > 0 && (!found_count || !order)) return fail(RBP_ERR_ARGUMENT, "rbp_queue_order: null buffer");
   const int cluster = B < CLUSTER_FROM ? 1 : CLUSTER;
-  RBP_CUDA(launch(order_kernel, cluster, cluster, static_cast<cudaStream_t>(stream), found_count, (long long)B, order,
-                  n_unsolved));
+  RBP_CUDA(launch(B < LARGE_FROM ? order_kernel<PER_SMALL> : order_kernel<PER_LARGE>, cluster, cluster,
+                  static_cast<cudaStream_t>(stream), found_count, (long long)B, order, n_unsolved));
   return RBP_OK;
 }
 

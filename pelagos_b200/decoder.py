@@ -791,18 +791,17 @@ class RelayBPDecoder:
     def _finish(self, raw: dict) -> Dict[str, torch.Tensor]:
         """The result dict of a launch's buffers (the unconverged-index list synchronises the host)."""
         found, iters, wfix = raw["found"], raw["iters"], raw["wfix"]
-        with torch.cuda.device(raw["gpu_id"]):
-            wdt = torch.float64 if self.dtype_str == "float64" else torch.float32
-            weights, valid, unconverged = finish_results(found, wfix, self.stop_nconv, wdt)
-            result = {
-                "errors": raw["packed"] if self.bitpack_output else raw["errors"],
-                "weights": weights,
-                "valid_mask": valid,
-                "iterations": iters,
-                "found_count": found,
-                "unconverged_indices": unconverged,
-                "weight_fixed": wfix,
-            }
-            if raw["last_post"] is not None:
-                result["last_posterior"] = raw["last_post"]
-            return result
+        wdt = torch.float64 if self.dtype_str == "float64" else torch.float32
+        weights, valid, unconverged = finish_results(found, wfix, self.stop_nconv, wdt)
+        result = {
+            "errors": raw["packed"] if self.bitpack_output else raw["errors"],
+            "weights": weights,
+            "valid_mask": valid,
+            "iterations": iters,
+            "found_count": found,
+            "unconverged_indices": unconverged,
+            "weight_fixed": wfix,
+        }
+        if raw["last_post"] is not None:
+            result["last_posterior"] = raw["last_post"]
+        return result

@@ -34,9 +34,9 @@ def test_results_and_order(B, share):
         assert int(count) == int((found <= 0).sum())
 
 
-# a cluster of 8 blocks from 32,768 shots on, a round being 16,384: around the change, parts of one round and of
-# several, blocks without a part, and a partial last round
+# rounds of 16,384 shots from 8,192 on, a cluster of 8 blocks from 32,768 on: around the changes, parts of one round
+# and of several, blocks without a part, and a partial last round
 @pytest.mark.parametrize("share", [0.0, 0.01, 1.0])
-@pytest.mark.parametrize("B", [16384, 16385, 32767, 32768, 32769, 131071, 131072, 131073, 262147, 600001])
+@pytest.mark.parametrize("B", [8191, 8192, 16384, 16385, 32767, 32768, 32769, 131071, 131072, 131073, 262147, 600001])
 def test_results_and_order_in_a_cluster(B, share):
     test_results_and_order(B, share)
