@@ -574,7 +574,7 @@ def run_mixed(args) -> None:
                                "[[144,12,12]] phenomenological p=0.003, (3,6)-regular 2000x4000 p=0.02",
                    "launch": mix.launch_info(), "autotuned_group_threads": tuned},
         "separate_launches": {"ms_per_step": ms_seq, "shots_per_s": 262144 / (ms_seq / 1000.0)},
-        "per_code": per_code, "gpu_launches": args.steps,
+        "per_code": per_code, "gpu_launches": args.steps * (1 + len(MIXED)),  # the decode, each code's result arrays
     }
     print(json.dumps(line), flush=True)
 

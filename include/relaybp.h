@@ -304,14 +304,18 @@ RBP_API int rbp_mixed_configure(rbp_mixed* m, const int32_t* group_threads);
  *     the alpha table [n_alpha] (may be NULL when use_alpha == 0);
  *   - the batch inputs and outputs, as for rbp_decode.
  * It decodes with the same kernel as rbp_decode, so the results are identical.
+ * It is not as fast: it does not see the values of an alpha table in device
+ * memory, so with one every check row takes the form that any alpha allows,
+ * and an edge keeps its place in its check's row, where a decoder chooses
+ * places against shared-memory bank conflicts.
  *
- * The graph tables it derives (check degrees, check pointers, slot positions)
+ * The graph tables it derives (check degrees, check pointers, slot positions, checks of a variable's edges)
  * and the kernel's work-queue counter live in a static device array of
  * RBP_STATIC_SCRATCH_BYTES bytes.  That array is part of the library image:
  * every GPU that loads the library holds it until the process exits.  A graph
  * whose tables need more returns RBP_ERR_UNSUPPORTED.  The call neither
  * allocates nor frees memory, on the device or on the host; it stages the
- * tables through a fixed stack buffer.
+ * tables through fixed stack buffers.
  *
  * All calls share that one array, and each call overwrites it: the counter is
  * cleared and every table is rewritten.  Calls that overlap on the GPU (on

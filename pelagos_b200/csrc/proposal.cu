@@ -21,17 +21,17 @@
 // ^ = rounded to bf16.  Weights are bf16 (an fp32 master copy is what AdamW
 // updates); every sum accumulates in fp32.
 //
-// Two implementations of the forward pass:
-//   * training kernels: one thread per output element, fp32, activations kept
-//     in device memory for the backward kernels (dense / gather / scatter
-//     forward and backward, loss, AdamW);
+// Three implementations of the forward pass:
+//   * training kernels: a thread owns one or two rows (checks of a shot), fp32 arithmetic, rounded layer
+//     inputs (bf16) and relu bits kept in device memory for the backward kernels; then loss, gradients, AdamW;
 //   * net_propose_kernel: the inference pass, one 512-thread block per SM
 //     looping over shots, with the graph, a shot's features, messages and
 //     per-variable sums in shared memory and the dense layers on the tensor
 //     cores (mma.sync m16n8k16 bf16 -> fp32).  A warp owns 16 checks at a
 //     time; the 64-wide node states g0/g1/g2 never leave its registers (they
-//     are recomputed from the saved 16-wide inputs x, a1, a2 instead of stored).
-// Both round at the same points, so they agree to fp32 summation order.
+//     are recomputed from the saved 16-wide inputs x, a1, a2 instead of stored);
+//   * net_propose_fast_kernel: the same pass, bit for bit, for graphs of low degrees.
+// All round at the same points, so training and inference agree to fp32 summation order.
 
 #include "relaybp.h"
 #include "relaybp_host.h"

@@ -10,9 +10,11 @@
 //   scan and the sign product run over all MAXDC slots without masks, and only
 //   rows that have padding put it back after their vector stores.
 // * The sign product is an XOR of the messages' raw bits (three operands per
-//   instruction); an output is (minimum) XOR (message's sign bit), the row's
-//   sign folded into the two candidate minima.
-// * min1/min2 by a tree of pairs: independent chains, four operations per merge.
+//   instruction); an output is its edge's minimum times +-alpha (+-1 without
+//   normalization), whose sign bit is the row's XOR the message's.
+// * Each edge's minimum over the other edges (min2 for a unique smallest, min1
+//   for the rest) comes from minima of pairs, quadruples and halves of the row,
+//   as three-input minima.
 // * 16-bit rows stay packed: two messages per instruction.
 // * The dummy slot of absent variable edges always holds 0, so sums need no
 //   mask; only the store to it is skipped.
@@ -30,8 +32,9 @@
 //     is NaN only when its memory mix is; float32 / bfloat16 variables then
 //     send +inf (edge_mix), which every other edge sees as the same thing.
 //     float16 messages saturate and cannot be NaN or inf.
-//   min1/min2: min(1e30, .) of the two smallest magnitudes; the cap is taken
-//     at the end, which only merges values that the cap makes equal anyway.
+//   min1/min2: min(1e30, .) of the two smallest magnitudes.  Here the cap is
+//     one more operand of the minima; a minimum does not depend on the order of
+//     its operands, so each edge receives min(1e30, the others) all the same.
 // An alpha table or beta that could make a check's output non-finite
 // (DevArgs::strict) runs the masked form; so do float64 rows.
 
