@@ -31,8 +31,9 @@ using rbph::fail;
 constexpr int FT = 1024;  // threads
 constexpr int CLUSTER = 8;
 // Shots per thread in a compacting block's round (PER): few where one round takes the batch, since a round's
-// instructions are the time then (order / results on the device, one shot: 4 per thread 2.4 / 2.0 us, 16 per
-// thread 4.7 / 3.3; 16,384 shots 8.3 / 4.1 and 8.4 / 4.1; in a cluster 32,768 take 10.2 / 7.5, in one block 14.4 / 6.5).
+// instructions are the time then.  Order / results on the device: one shot 2.1 / 1.7 us (with 16 per thread, and
+// the parts' sizes in 64 bits, 4.7 / 3.3), 16,384 shots 8.0 / 3.9, 32,768 and 65,536 in a cluster 9.9 / 6.8 (32,768
+// in one block 14.4 / 6.5).
 constexpr int PER_SMALL = 4, PER_LARGE = 16;
 constexpr int64_t LARGE_FROM = 2 * PER_SMALL * FT;
 constexpr int64_t CLUSTER_FROM = 2 * PER_LARGE * FT;
@@ -43,8 +44,9 @@ struct Part {
 };
 template <int PER>
 __device__ __forceinline__ Part part_of(long long B, unsigned rank, unsigned n) {
-  const long long rounds = (B + PER * FT - 1) / (PER * FT), each = (rounds + n - 1) / n * (PER * FT);
-  const long long i0 = min(B, each * rank);
+  if (n == 1) return {0, B};
+  const unsigned rounds = (unsigned)((B + PER * FT - 1) / (PER * FT));
+  const long long each = (long long)((rounds + n - 1) / n) * (PER * FT), i0 = min(B, each * rank);
   return {i0, min(B, i0 + each)};
 }
 
